@@ -79,7 +79,8 @@ struct ccs_handle {
     std::string kind_name;
     ccs::KindDesc kind;
     bool kind_ready = false;
-    ccs::DevTables* d_tables = nullptr;
+    ccs::DevImage* d_image = nullptr;     // the kind's constants
+    ccs::DevTables* d_tables = nullptr;   // ... of most kernels (in d_image)
     uint32_t* d_classidx = nullptr;
     uint32_t* d_class_rep = nullptr;
     uint16_t* d_class_stab = nullptr;

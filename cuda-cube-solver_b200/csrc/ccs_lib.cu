@@ -134,7 +134,8 @@ int set_kind(ccs_handle* h, const char* name) {
     if (h->kind_ready && h->kind_name == name) return CCS_OK;
     CUDA_TRY(cudaSetDevice(h->device));
     if (!h->d_tables) {
-        CUDA_TRY(cudaMalloc(&h->d_tables, sizeof(DevTables)));
+        CUDA_TRY(cudaMalloc(&h->d_image, sizeof(DevImage)));
+        h->d_tables = &h->d_image->t;
         const CornerClasses& cc = corner_classes();
         CUDA_TRY(cudaMalloc(&h->d_classidx, cc.classidx.size() * 4));
         CUDA_TRY(cudaMalloc(&h->d_class_rep, cc.rep.size() * 4));
@@ -143,9 +144,10 @@ int set_kind(ccs_handle* h, const char* name) {
         CUDA_TRY(cudaMemcpy(h->d_class_rep, cc.rep.data(), cc.rep.size() * 4, cudaMemcpyHostToDevice));
         CUDA_TRY(cudaMemcpy(h->d_class_stab, cc.stab.data(), cc.stab.size() * 2, cudaMemcpyHostToDevice));
     }
-    auto T = std::make_unique<DevTables>();
-    build_dev_tables(k, T.get());
-    CUDA_TRY(cudaMemcpy(h->d_tables, T.get(), sizeof(DevTables), cudaMemcpyHostToDevice));
+    auto T = std::make_unique<DevImage>();
+    build_dev_tables(k, &T->t);
+    build_warp_tables(T->t, &T->w);
+    CUDA_TRY(cudaMemcpy(h->d_image, T.get(), sizeof(DevImage), cudaMemcpyHostToDevice));
     h->kind = k;
     h->kind_name = name;
     h->kind_ready = true;
@@ -205,7 +207,7 @@ int ccs_close(ccs_handle* h) {
     cudaSetDevice(h->device);
     if (h->server) server_stop(h);
     free_table(h);
-    cudaFree(h->d_tables);
+    cudaFree(h->d_image);
     cudaFree(h->d_classidx);
     cudaFree(h->d_class_rep);
     cudaFree(h->d_class_stab);

@@ -332,10 +332,11 @@ __device__ __forceinline__ void unrank_dev(const DevTables& T, const uint32_t* _
 
 // Copy the constant tables into shared memory (whole block).
 #ifndef CCS_HOST_EMULATION
-__device__ __forceinline__ void stage_tables(DevTables& dst, const DevTables* __restrict__ src) {
+template <class Tables>
+__device__ __forceinline__ void stage_tables(Tables& dst, const Tables* __restrict__ src) {
     const uint4* s = reinterpret_cast<const uint4*>(src);
     uint4* d = reinterpret_cast<uint4*>(&dst);
-    for (int i = threadIdx.x; i < (int)(sizeof(DevTables) / 16); i += blockDim.x) d[i] = s[i];
+    for (int i = threadIdx.x; i < (int)(sizeof(Tables) / 16); i += blockDim.x) d[i] = s[i];
     __syncthreads();
 }
 #endif

@@ -139,4 +139,41 @@ void build_dev_tables(const KindDesc& kind, DevTables* T) {
     }
 }
 
+void build_warp_tables(const DevTables& t, WarpTables* W) {
+    std::memset(W, 0, sizeof(WarpTables));
+    for (int m = 0; m < 18; ++m) {
+        uint32_t* r = W->right[m];
+        for (int w = 0; w < 2; ++w) r[w] = t.mv_csel[m][w], r[2 + w] = t.mv_cadd[m][w];
+        for (int w = 0; w < 3; ++w)
+            r[4 + w] = t.mv_esel[m][w], r[7 + w] = t.mv_esel2[m][w], r[10 + w] = t.mv_emsk[m][w], r[13 + w] = t.mv_eflp[m][w];
+        for (int w = 0; w < 2; ++w) W->left[m][w] = t.lf_c[m][w];
+        for (int w = 0; w < 3; ++w) W->left[m][2 + w] = t.lf_e[m][w];
+        for (int k = 0; k < 3; ++k) {
+            W->act[k][m] = t.frame_move[k][m];
+            W->act[3 + k][m] = t.inv_move[t.frame_move[k][m]];
+        }
+    }
+    for (int s = 0; s < 16; ++s) {
+        for (int w = 0; w < 3; ++w) W->sym[s][w] = t.sy_psel[s][w];
+        W->sym[s][3] = t.sy_fx[s] ? 256u | (512u << 16) : 0u;
+        W->swap[s] = t.sy_swap[s];
+    }
+    for (int em = 0; em < 16; ++em)
+        for (int x = 0; x < 16; ++x) {
+            const int n = __builtin_popcount(em), i = em | (x << 4);
+            W->flp[0][i] = (uint16_t)(t.flp[(em << 4) | x] | (n << 8));
+            W->flp[1][i] = (uint16_t)(t.flp[(em << 4) | (x ^ em)] | (n << 8));
+            W->flp[2][i] = (uint16_t)(t.flp[(em << 4) | (x ^ em ^ 15)] | (n << 8));
+            W->ump[0][i] = t.ump[(em << 4) | x];
+            W->ump[1][i] = t.ump[(em << 4) | (x ^ 15)];
+        }
+    std::memcpy(W->slice_rank, t.slice_rank, sizeof W->slice_rank);
+    std::memcpy(W->genc[0], t.genc, sizeof t.genc);
+    std::memcpy(W->genc[1], t.genc2, sizeof t.genc2);
+    std::memcpy(W->lab, t.sy_lab, sizeof W->lab);
+    std::memcpy(W->cmp4, t.cmp4, sizeof W->cmp4);
+    std::memcpy(W->ccomb_rank, t.ccomb_rank, sizeof W->ccomb_rank);
+    std::memcpy(W->amask, t.amask, sizeof W->amask);
+}
+
 }  // namespace ccs

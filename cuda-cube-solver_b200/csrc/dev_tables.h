@@ -53,6 +53,33 @@ struct alignas(16) DevTables {
     uint32_t amask[20];          // canonical successors of last move (index last + 1), 18 bits
 };
 
+// What the warp search kernel stages instead (warp_tables.cuh): the same content in rows that one or
+// a few 128-bit loads bring, padded so that lanes on different rows meet few bank conflicts.
+struct alignas(16) WarpTables {
+    uint32_t right[18][20];      // csel[2] cadd[2], esel[3], esel2[3], emsk[3], eflp[3], padding
+    uint32_t left[18][12];       // lf_c[2] lf_e[3], padding
+    uint32_t sym[16][4];         // sy_psel[3], flp row offsets: words 0 and 1 | word 2 << 16
+    uint16_t slice_rank[4096];
+    uint16_t flp[3][256];        // E mask4 | flip mask4 << 4: see warp_edge_coord; rows: flips as they
+                                 // are, flips ^ E mask, flips ^ ~E mask
+    uint16_t genc[2][384];       // E-content classes of the first and the second resident table
+    uint8_t lab[16][256];        // sy_lab
+    uint8_t cmp4[16][256];
+    uint8_t ump[2][256];         // E mask4 | U mask4 << 4 -> U mask over the others; [1]: complemented
+    uint8_t ccomb_rank[256];
+    uint8_t act[6][32];          // move m of the cube as a row of `right` (frames 0-2) or `left` (3-5)
+    uint8_t swap[16];
+    uint32_t amask[20];
+};
+
+// Device image of a kind's constants.
+struct DevImage {
+    DevTables t;
+    WarpTables w;
+};
+
+void build_warp_tables(const DevTables& t, WarpTables* out);
+
 // Fills the tables for a kind (gen tables from KindDesc; unused for KIND_304); genc2 starts as a
 // copy of genc.
 void build_dev_tables(const KindDesc& kind, DevTables* out);
@@ -62,4 +89,5 @@ void build_genc(const KindDesc& kind, uint16_t genc[384]);
 
 }  // namespace ccs
 
+static_assert(sizeof(ccs::WarpTables) % 16 == 0, "WarpTables is staged with 16-byte copies");
 static_assert(sizeof(ccs::DevTables) % 16 == 0, "DevTables is staged with 16-byte copies");

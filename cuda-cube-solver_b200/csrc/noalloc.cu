@@ -218,6 +218,8 @@ extern "C" int ccs_solve_noalloc(ccs_handle* h, const uint32_t* states, int n, c
     CCS_CUDA_TRY(cudaMemcpyAsync(D.slots, S->slots, sizeof(Slot) * n, cudaMemcpyDeviceToHost, st));
     CCS_CUDA_TRY(cudaStreamSynchronize(st));
     for (int i = 0; i < n; ++i) fill_result(D.slots[i], &results[i]);
+    if (q.error & (ERR_STACK | ERR_STUCK))
+        return fail(CCS_E_CHECK, "a search ran out of room for its nodes (error bits %u)", q.error);
     if (q.error & ERR_BOUND) return fail(CCS_E_CHECK, "a search passed the largest possible bound");
     return CCS_OK;
 }

@@ -71,7 +71,7 @@ struct alignas(32) DonationCell {
 };
 constexpr uint32_t DON_EMPTY = 0, DON_WRITING = 1, DON_FULL = 2, DON_READING = 3;
 
-constexpr uint32_t ERR_IDLE_LIMIT = 1u, ERR_BOUND = 2u, ERR_STACK = 4u;
+constexpr uint32_t ERR_IDLE_LIMIT = 1u, ERR_BOUND = 2u, ERR_STACK = 4u, ERR_STUCK = 8u;
 
 struct SearchParams {
     Slot* slots;
@@ -93,6 +93,9 @@ struct SearchParams {
     uint32_t shallow_min_active;     // ... applied only while at least this many cubes are active
     uint32_t few_max_active;         // with at most this many cubes in flight ...
     uint32_t few_divisor;            // ... the deeper thresholds are divided by this
+    uint32_t warp_items;             // 1: items are for whole warps (shorter prefixes, see next_plen)
+    unsigned long long warp_at[2];   // ... an iteration of at least this many nodes -> one move longer,
+    unsigned long long warp_many_at[2];  // ... with many cubes in flight
     uint32_t idle_limit;             // idle polls before a warp leaves (kernel relaunched by the host)
     uint32_t spread;                 // lanes take items from up to this many queued iterations
     uint32_t move_min;               // phased kernel: lanes waiting before a MOVE pass runs

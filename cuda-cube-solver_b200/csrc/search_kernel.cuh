@@ -24,9 +24,13 @@
 namespace ccs {
 
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
+#ifdef CCS_HOST_EMULATION
+    return 0;
+#else
     unsigned long long t;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
     return t;
+#endif
 }
 
 __device__ __forceinline__ uint32_t hget(uint32_t h, int k) { return (h >> (5 * k)) & 31u; }
@@ -154,7 +158,13 @@ __device__ __forceinline__ uint32_t next_plen(const SearchParams& P, unsigned lo
     const unsigned long long d1 = few ? P.deeper_at[1] / P.few_divisor : P.deeper_at[1];
     // signed: a base of 1 minus two shallow steps is -1, clamped to 1 (never a wrapped length)
     int pl = (int)P.base_plen + (int)(last_nodes >= d0) + (int)(last_nodes >= d1);
-    if (many) pl -= (int)(last_nodes < P.shallow_at[0]) + (int)(last_nodes < P.shallow_at[1]);
+    if (P.warp_items) {
+        // an item is searched by a warp: two moves shorter than for a lane, one longer per threshold
+        const unsigned long long* at = many ? P.warp_many_at : P.warp_at;
+        pl += (int)(last_nodes >= at[0]) + (int)(last_nodes >= at[1]) - 2;
+    } else if (many) {
+        pl -= (int)(last_nodes < P.shallow_at[0]) + (int)(last_nodes < P.shallow_at[1]);
+    }
     const int top = (int)P.max_plen;  // the longest prefix length with a list in this launch
     pl = pl < 1 ? 1 : (pl > top ? top : pl);
     return (uint32_t)pl < bound ? (uint32_t)pl : bound;
@@ -233,7 +243,8 @@ __device__ __forceinline__ bool server_idle(const SearchParams& P) {
 // one long-lived entry; with P.head_limit 0 the limit is half the ring.
 static __device__ __noinline__ void advance_head(const SearchParams& P) {
     volatile QueueState* q = P.q;
-    const unsigned long long limit = P.head_limit ? P.head_limit : P.ring_cap / 2u;
+    // (never past half the ring: a live entry at the head would be overwritten when the ring wraps)
+    const unsigned long long half = P.ring_cap / 2u, limit = P.head_limit && P.head_limit < half ? P.head_limit : half;
     for (int a = 0; a < 4; ++a) {
         unsigned long long h = q->head, t = q->tail;
         if (h >= t) return;
@@ -339,16 +350,24 @@ __device__ __forceinline__ uint32_t probe_bound(const DevTables& T, const Search
     return probe_dev<MODE, NEC, FMT>(T, P.classidx, second ? P.table2 : P.table, s, second);
 }
 
+// Root frame k of a cube.  Slots are read past the L1 (here and wherever a root frame, h0 or the table
+// is read): a server reuses a slot while the launch runs, and the L1 of an SM that searched the last
+// cube in it may still hold that cube's lines.
+__device__ __forceinline__ State slot_frame(const Slot& sl, uint32_t k) {
+    const uint32_t* f = sl.frame + 5u * k;
+    return State{__ldcg(f), __ldcg(f + 1), __ldcg(f + 2), __ldcg(f + 3), __ldcg(f + 4)};
+}
+
 // Admission of a new cube: root bounds of its six frames, first threshold, first iteration.
 template <int MODE, int NEC, int FMT>
 __device__ void admit_slot(const DevTables& T, const SearchParams& P, uint32_t s) {
     Slot& sl = P.slots[s];
-    State f0{sl.frame[0], sl.frame[1], sl.frame[2], sl.frame[3], sl.frame[4]};
-    const bool second = sl.table != 0u;
+    const State f0 = slot_frame(sl, 0u);
+    const bool second = __ldcg(&sl.table) != 0u;
     uint32_t h = 0, bound = 0;
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
-        State f{sl.frame[5 * k], sl.frame[5 * k + 1], sl.frame[5 * k + 2], sl.frame[5 * k + 3], sl.frame[5 * k + 4]};
+        const State f = slot_frame(sl, (uint32_t)k);
         uint32_t v = probe_bound<MODE, NEC, FMT>(T, P, f, second);
         v = v > 31u ? 31u : v;
         h = hset(h, k, v);
@@ -383,7 +402,7 @@ struct FramesReg {
     __device__ __forceinline__ State first() const { return f[0]; }
     __device__ __forceinline__ void load(const uint32_t* src) {
 #pragma unroll
-        for (int j = 0; j < 6; ++j) f[j] = State{src[5 * j], src[5 * j + 1], src[5 * j + 2], src[5 * j + 3], src[5 * j + 4]};
+        for (int j = 0; j < 6; ++j) f[j] = State{__ldcg(src + 5 * j), __ldcg(src + 5 * j + 1), __ldcg(src + 5 * j + 2), __ldcg(src + 5 * j + 3), __ldcg(src + 5 * j + 4)};
     }
     __device__ __forceinline__ void step(const DevTables& T, int m) {
 #pragma unroll
@@ -414,7 +433,7 @@ struct FramesSmem {
     __device__ __forceinline__ State first() const { return get(0); }
     __device__ __forceinline__ void load(const uint32_t* src) {
 #pragma unroll
-        for (int i = 0; i < 30; ++i) w[i * THREADS] = src[i];
+        for (int i = 0; i < 30; ++i) w[i * THREADS] = __ldcg(src + i);
     }
     __device__ __forceinline__ void step(const DevTables& T, int m) {
 #pragma unroll
@@ -522,7 +541,7 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel(const DevTables* 
                     continue;
                 }
 f.load(sl.frame);
-                h = sl.h0;
+                h = __ldcg(&sl.h0);
                 pseq = plen ? __ldg(P.prefixes[plen] + idx) : 0u;
                 g = 0;
                 last = -1;

@@ -6,6 +6,7 @@
 #include "dispatch.cuh"
 #include "search_kernel.cuh"
 #include "search_phased.cuh"
+#include "search_warp.cuh"
 
 namespace ccs {
 
@@ -29,11 +30,24 @@ int launch_phased(ccs_handle* h, const SearchParams& P, int grid, cudaStream_t s
     return CCS_OK;
 }
 
-// Kernel variants (ccs_solve_opts.variant, resolved 1..11): see resolve_variant in solve.cu.
+constexpr int WARP_THREADS = 640;  // 20 warps per SM, in one block (see search_warp.cuh)
+
+template <int MODE, int NEC, int FMT, int THREADS, int MINB>
+int launch_warp(ccs_handle* h, const SearchParams& P, int grid, cudaStream_t stream) {
+    auto* k = search_kernel_warp<MODE, NEC, FMT, THREADS, MINB>;
+    constexpr size_t dyn = warp_dyn_smem<THREADS>();
+    CCS_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    k<<<grid, THREADS, dyn, stream>>>(&h->d_image->w, P);
+    CCS_CUDA_TRY(cudaGetLastError());
+    return CCS_OK;
+}
+
+// Kernel variants (ccs_solve_opts.variant, resolved 1..12): see resolve_variant in solve.cu.
 template <int MODE, int NEC>
 int launch_kind(ccs_handle* h, const SearchParams& P, int grid, cudaStream_t stream, int variant) {
     return dispatch_fmt(h->format, [&](auto F) {
         constexpr int FMT = decltype(F)::value;
+        if (variant == 12) return launch_warp<MODE, NEC, FMT, WARP_THREADS, 1>(h, P, grid, stream);
         if (variant == 2) return launch_phased<MODE, NEC, FMT, 256, 2, true>(h, P, grid, stream);
         if (variant == 3) return launch_phased<MODE, NEC, FMT, 256, 3>(h, P, grid, stream);
         if (variant == 4) return launch_variant<MODE, NEC, FMT, 256, false, 2>(h, P, grid, stream);
@@ -56,7 +70,8 @@ int kernel_footprint_kind(ccs_handle* h, int variant, size_t* local_bytes, int* 
         cudaFuncAttributes a{};
         int t = 256;
         cudaError_t e;
-        if (variant == 2) e = cudaFuncGetAttributes(&a, search_kernel_phased<MODE, NEC, FMT, 256, 2, true>);
+        if (variant == 12) e = (t = WARP_THREADS, cudaFuncGetAttributes(&a, search_kernel_warp<MODE, NEC, FMT, WARP_THREADS, 1>));
+        else if (variant == 2) e = cudaFuncGetAttributes(&a, search_kernel_phased<MODE, NEC, FMT, 256, 2, true>);
         else if (variant == 3) e = cudaFuncGetAttributes(&a, search_kernel_phased<MODE, NEC, FMT, 256, 3>);
         else if (variant == 4) e = cudaFuncGetAttributes(&a, search_kernel<MODE, NEC, FMT, 256, false, 2>);
         else if (variant == 5) e = (t = 512, cudaFuncGetAttributes(&a, search_kernel<MODE, NEC, FMT, 512, true, 2>));

@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_phased(const DevT
                         path[j] = (unsigned char)mj;
                         f.step(T, mj);
                     }
-                    second = sl.table != 0u;
+                    second = __ldcg(&sl.table) != 0u;
                     h = (uint32_t)w1 & 0x3FFFFFFFu;
                     g = gbase = g0;
                     plen = 0;
@@ -220,8 +220,8 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_phased(const DevT
                     have = true;
                 } else {
                     f.load(sl.frame);
-                    second = sl.table != 0u;
-                    h = sl.h0;
+                    second = __ldcg(&sl.table) != 0u;
+                    h = __ldcg(&sl.h0);
                     pseq = plen ? __ldg(P.prefixes[plen] + idx) : 0u;
                     g = 0;
                     nodes = 0;

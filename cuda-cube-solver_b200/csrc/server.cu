@@ -39,7 +39,7 @@ struct Server {
     bool kernel_running = false;
     SearchParams P{};
     int grid = 0;
-    int variant = 3;  // resolved kernel variant
+    int variant = 12;  // resolved kernel variant
     unsigned long long* done_log = nullptr;  // host-mapped
     unsigned long long* d_done_log = nullptr;
     uint32_t log_cap = 0;
@@ -178,12 +178,9 @@ constexpr uint32_t SERVER_MAX_SLOTS = 65536;
 template <int MODE, int NEC>
 int kernel_footprint_kind(ccs_handle* h, int variant, size_t* local_bytes, int* threads);
 
-// The automatic server shape is 256 x 2 with sibling lookahead (variant 2), the low-latency one:
-// on B200 a stream at 10 requests/s has a p50 of 21 ms with it and 46 ms with 256 x 3; at 100
-// requests/s (90% uniform, 9% of length >= 18, 1% superflips) 256 x 3 is ahead (91 cubes/s
-// sustained, p50 94 ms, against 87-89 cubes/s, p50 123-165 ms).
+// The automatic server kernel is the solve calls' (variant 12).
 static int server_variant(const ccs_solve_opts* opts) {
-    return opts && opts->variant > 0 ? resolve_variant(opts, 0) : 2;
+    return resolve_variant(opts, 0);
 }
 
 // Device memory the server holds whatever the number of cubes: resident tables, constants,
@@ -198,7 +195,7 @@ int server_fixed_bytes(ccs_handle* h, const ccs_solve_opts* opts, uint64_t* out)
     }));
     uint64_t prefixes = 0;
     for (int L = 0; L <= MAX_PLEN; ++L) prefixes += 4ull * h->n_prefix[L];
-    *out = h->table_bytes + h->table2_bytes + sizeof(DevTables) + 153090ull * 4 + 9930ull * 6 + prefixes +
+    *out = h->table_bytes + h->table2_bytes + sizeof(DevImage) + 153090ull * 4 + 9930ull * 6 + prefixes +
            sizeof(QueueState) + sizeof(DonationCell) * DON_CELLS + (uint64_t)local * threads * grid;
     return CCS_OK;
 }

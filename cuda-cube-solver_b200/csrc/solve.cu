@@ -42,6 +42,8 @@ int ensure_search_buffers(ccs_handle* h, uint32_t slots) {
     return CCS_OK;
 }
 
+int resolve_variant(const ccs_solve_opts* o, int cubes);
+
 void fill_params(ccs_handle* h, const ccs_solve_opts* o, SearchParams* P) {
     std::memset(P, 0, sizeof *P);
     P->slots = h->d_slots;
@@ -91,6 +93,22 @@ void fill_params(ccs_handle* h, const ccs_solve_opts* o, SearchParams* P) {
     P->don_eager = o && o->steal == 2 ? 0u : 1u;
     P->don_min_prev = o && o->steal_min_nodes != 0 ? (o->steal_min_nodes > 0 ? (unsigned long long)o->steal_min_nodes : 0ull)
                                                    : 10000000ull;
+    // The warp kernel (variant 12): an item is searched by 32 lanes, so its prefix is two moves shorter
+    // to begin with and grows with the last iteration's nodes -- an item of a few hundred nodes
+    // keeps a warp busy past the walk to it, and 2,960 warps need some items each.  With many cubes
+    // in flight other cubes fill the warps, and longer items cost fewer walks.
+    P->warp_items = resolve_variant(o, 0) == 12 ? 1u : 0u;
+    P->warp_at[0] = 20000ull;
+    P->warp_at[1] = 200000ull;
+    P->warp_many_at[0] = 300000ull;
+    P->warp_many_at[1] = 30000000ull;
+    if (P->warp_items) {
+        // Donations are cheap (an entry of the warp's stack), so they start with small iterations and
+        // are looked for often; the deeper thresholds are not divided for few cubes.
+        if (!(o && o->steal_min_nodes != 0)) P->don_min_prev = 10000ull;
+        if (!(o && o->steal_period > 0)) P->don_period = 16u;
+        if (!(o && o->few_divisor > 0)) P->few_divisor = 1u;
+    }
     // Head rotation at half the scan window (rotate 1) or at half the ring (-1, the batch default).
     P->head_limit = o && o->rotate > 0 ? std::max<unsigned long long>(P->spread / 2u, 32u) : 0ull;
     P->done_log = nullptr;
@@ -105,13 +123,12 @@ void fill_params(ccs_handle* h, const ccs_solve_opts* o, SearchParams* P) {
 // 6 = phase-ordered, 128 x 4 (4 warps per block); 7 = phase-ordered, 512 x 1 (16 warps per block);
 // 8 = sibling lookahead, 256 x 3; 9 = phase-ordered, 256 x 4 (32 warps per SM, 64 registers);
 // 10 = phase-ordered, 224 x 3 (21 warps, 96 registers); 11 = phase-ordered, 128 x 5 (20 warps, 96).
-// 0 = automatic: 2 for fewer than 64 cubes, else 3 (and 3 for the server).  Measured on B200
-// (d4t, 1,024 uniform cubes): 3 reaches 338 cubes/s (31.0 G probes/s) against 283 for 1 and 292
-// for 2 -- its 80-register cap spills a little, to an L1 that the table sectors no longer
-// occupy; a lone cube is faster on 2 (plain 1-cube p50 16.6 ms against 25.0 ms).
+// 12 = one search per warp (search_warp.cuh), 640 x 1.  0 = automatic: 12.  Measured on B200 (d4t,
+// cubes/s at one cube per call / 16 / 100 / 1,024 per call): 12 155 / 260 / 300 / 351, 2 58 / 131 /
+// 179 / 275, 3 44 / 125 / 162 / 334.
 int resolve_variant(const ccs_solve_opts* o, int cubes) {
     int v = o ? o->variant : 0;
-    if (v <= 0 || v > 11) v = cubes > 0 && cubes < 64 ? 2 : 3;
+    if (v <= 0 || v > 12) v = 12;
     return v;
 }
 
@@ -120,7 +137,7 @@ int grid_for(ccs_handle* h, const ccs_solve_opts* o, int variant) {
                                          : (variant == 3 || variant == 8 || variant == 10 ? 3
                                           : variant == 6 || variant == 9 ? 4
                                           : variant == 11 ? 5
-                                          : variant == 7 ? 1 : 2);
+                                          : variant == 7 || variant == 12 ? 1 : 2);
     return bps * h->sms;
 }
 
@@ -129,7 +146,7 @@ int grid_for(ccs_handle* h, const ccs_solve_opts* o, int variant) {
 template <int MODE, int NEC>
 int launch_kind(ccs_handle* h, const SearchParams& P, int grid, cudaStream_t stream, int variant);
 
-// variant: a resolved one (1..7).
+// variant: a resolved one (1..12).
 int launch_kernel(ccs_handle* h, const SearchParams& P, int grid, cudaStream_t stream, int variant) {
     return dispatch_kind(h->kind, [&](auto M, auto N) {
         return launch_kind<decltype(M)::value, decltype(N)::value>(h, P, grid, stream, variant);
@@ -193,7 +210,7 @@ extern "C" int ccs_solve_tables(ccs_handle* h, const uint32_t* states, const uin
     SearchParams P;
     fill_params(h, opts, &P);
     P.n_slots = (uint32_t)n;
-    if (n < 64) {
+    if (!P.warp_items && n < 64) {
         // Few cubes per call (the plain drop-in's shape) have their own defaults: a push or pop
         // runs as soon as one lane waits for it, a probe pass repeats while 8 lanes probe, and
         // deeper prefixes start 200x sooner while at most 4 cubes are in flight.  Measured on
@@ -250,6 +267,8 @@ extern "C" int ccs_solve_tables(ccs_handle* h, const uint32_t* states, const uin
     CCS_CUDA_TRY(cudaMemcpyAsync(host.data(), h->d_slots, sizeof(Slot) * n, cudaMemcpyDeviceToHost, st));
     CCS_CUDA_TRY(cudaStreamSynchronize(st));
     for (int i = 0; i < n; ++i) fill_result(host[i], &results[i]);
+    if (q.error & (ERR_STACK | ERR_STUCK))
+        return fail(CCS_E_CHECK, "a search ran out of room for its nodes (error bits %u)", q.error);
     if (q.error & ERR_BOUND) return fail(CCS_E_CHECK, "a search passed the largest possible bound");
     return CCS_OK;
 }

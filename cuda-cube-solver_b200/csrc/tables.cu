@@ -161,6 +161,8 @@ static int attach_second(ccs_handle* h, const char* kind, int format, uint32_t* 
     build_genc(k2, genc);
     CCS_CUDA_TRY(cudaMemcpy(reinterpret_cast<char*>(h->d_tables) + offsetof(DevTables, genc2), genc, sizeof genc,
                             cudaMemcpyHostToDevice));
+    CCS_CUDA_TRY(cudaMemcpy(reinterpret_cast<char*>(h->d_image) + offsetof(DevImage, w) + offsetof(WarpTables, genc) + sizeof genc,
+                            genc, sizeof genc, cudaMemcpyHostToDevice));
     if (h->d_table2) cudaFree(h->d_table2);
     h->d_table2 = d;
     h->table2_bytes = bytes;

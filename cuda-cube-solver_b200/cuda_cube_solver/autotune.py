@@ -3,17 +3,17 @@ GPU, table and batch size by measuring them.
 
 Knobs (``native.SolveOpts``):
 
-* ``variant``: search kernel and launch shape -- 3 = 256 threads x 3 blocks per SM (the batched
-  default), 1 = 256 x 2, 2 = 256 x 2 with sibling lookahead (two probe chains per lane), 8 =
+* ``variant``: search kernel and launch shape -- 12 = one search per warp, 640 threads per SM (the
+  default); one search per lane: 3 = 256 threads x 3 blocks per SM, 1 = 256 x 2, 2 = 256 x 2 with sibling lookahead (two probe chains per lane), 8 =
   lookahead 256 x 3, 10 = 224 x 3, 11 = 128 x 5, 6 = 128 x 4 (4 warps per block), 7 = 512 x 1
   (16 warps per block), 9 = 256 x 4 (32 warps per SM);
 * ``base_plen``: cut depth of the work items (prefix length of a cube's iterations), 3-6;
-* ``move`` = (``move_min``, ``move_age``): how many lanes wait, and for how many iterations,
+* ``move`` = (``move_min``, ``move_age``) (variants 1-11): how many lanes wait, and for how many iterations,
   before the frame-update pass (push / pop) runs -- the depth of the lanes' update pipeline, 1-16;
 * ``steal_depth``: the least slack (moves to the bound beyond a node's largest frame bound) of a
   node whose children a lane donates to idle lanes;
 * ``spread``: over how many queued cubes the lanes spread;
-* ``probe_min``: a warp keeps probing while at least this many lanes have a probe.
+* ``probe_min`` (variants 1-11): a warp keeps probing while at least this many lanes have a probe.
 
 Coordinate descent from the library defaults: each knob in turn takes the value with the best
 device time on the sample (the same cubes every time), within a time budget; a value replaces the
@@ -35,14 +35,14 @@ from cuda_cube_solver.device import state_words
 CACHE = Path(os.environ.get("CCS_TUNE_CACHE", Path.home() / ".cache" / "cuda_cube_solver" / "autotune.json"))
 
 SPACE = {
-    "variant": [3, 1, 2, 8, 10, 11, 6, 7, 9],
+    "variant": [12, 3, 1, 2, 8, 10, 11, 6, 7, 9],
     "base_plen": [3, 4, 5, 6],
     "move": [(1, 1), (4, 2), (8, 4), (16, 8)],
     "steal_depth": [1, 2, 3, 4],
     "spread": [512, 1024, 4096],
     "probe_min": [12, 16, 20, 24],
 }
-DEFAULT = {"variant": 3, "base_plen": 4, "move": (8, 4), "steal_depth": 2, "spread": 4096, "probe_min": 16}
+DEFAULT = {"variant": 12, "base_plen": 4, "move": (8, 4), "steal_depth": 2, "spread": 4096, "probe_min": 16}
 MIN_GAIN = 0.02  # a setting must cut the sample's device time by 2% to replace the incumbent
 
 

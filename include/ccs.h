@@ -162,10 +162,14 @@ typedef struct ccs_solve_opts {
     int threads;              /* threads per block: 128, 256 or 512 (0: default)            */
     double timeout_s;         /* give up after this long (0: no limit)                      */
     int spread;               /* lanes work on up to this many queued cubes at once (0: 4096) */
-    int variant;              /* search kernel: 0 automatic (2 below 64 cubes, else 3), 1 = 256 */
-                              /*   threads x 2 blocks/SM, 2 = sibling lookahead (two probe      */
-                              /*   chains per lane), 3 = 256 x 3, 6 = 128 x 4, 7 = 512 x 1,      */
-                              /*   8 = lookahead 256 x 3 (4-5: loop-control forms)              */
+    int variant;              /* search kernel: 0 automatic (12), 12 = one search per warp,     */
+                              /*   640 threads x 1 block/SM; one search per lane: 1 = 256 x 2,  */
+                              /*   2 = sibling lookahead (two probe chains per lane), 3 = 256   */
+                              /*   x 3, 6 = 128 x 4, 7 = 512 x 1, 8 = lookahead 256 x 3, 9 =    */
+                              /*   256 x 4, 10 = 224 x 3, 11 = 128 x 5 (4-5: loop-control       */
+                              /*   forms).  12 starts an item at base_plen - 2 moves, and one   */
+                              /*   or two more as iterations grow; it has no use for            */
+                              /*   shallow_at, move_min, move_age and probe_min.                */
     double shallow_at0;       /* an iteration of < this many nodes makes the next one use a    */
     double shallow_at1;       /*   prefix one move shorter (0: 1e5 / 1.5e6, < 0: off)          */
     int move_min;             /* lanes waiting before a frame-update pass runs (0: 8; 1 in a   */
@@ -181,13 +185,15 @@ typedef struct ccs_solve_opts {
     int steal_depth;          /* a donated node's slack -- moves to the bound beyond its largest */
                               /*   frame bound -- is at least this (0: 2)                       */
     int steal_period;         /* a lane with work checks for starving lanes every this many    */
-                              /*   iterations, a power of two (0: 64)                           */
+                              /*   iterations, a power of two (0: 64; 16 in variant 12)         */
     int steal_target;         /* donors stop once this many subtrees wait (0: 512)              */
     int few_divisor;          /* while at most 4 cubes are in flight, deeper_at0/1 are divided */
                               /*   by this (0: 50, or 200 in a ccs_solve of fewer than 64       */
-                              /*   cubes; 1: never, the reference's plain thresholds)           */
+                              /*   cubes, or 1 in variant 12; 1: never, the reference's plain   */
+                              /*   thresholds)                                                  */
     double steal_min_nodes;   /* subtrees of a cube are donated only once its previous          */
-                              /*   iteration reached this many nodes (0: 1e7; < 0: always)      */
+                              /*   iteration reached this many nodes (0: 1e7, or 1e4 in variant */
+                              /*   12; < 0: always)                                             */
     int rotate;               /* a live entry at the work ring's head moves to the tail once   */
                               /*   the queue spans half of `spread` (1), or half the ring (-1), */
                               /*   so every queued cube stays within the lanes' scan window     */

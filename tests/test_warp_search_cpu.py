@@ -1,0 +1,71 @@
+"""The warp search kernel on the host (tests/emul/warp_emul.cpp): its probe arithmetic against the CPU
+oracle for every kind, and whole searches of one emulated warp on an all-zero table, at full size and
+with so few nodes and stash entries that the spill list carries most of the search."""
+
+from __future__ import annotations
+
+import ctypes
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import ROOT
+from cuda_cube_solver import workloads
+from cuda_cube_solver.cubie import MOVES_HTM, CubieState, apply_moves
+from cuda_cube_solver.device import state_words
+from cuda_cube_solver.prefixes import canonical_prefixes
+
+KINDS = ["304", "s4", "d4f", "a4t", "d4t", "d4", "a4"]
+
+
+@pytest.fixture(scope="module")
+def libs():
+    subprocess.run(["make", "-C", str(ROOT / "tests" / "emul"), "warp"], check=True, capture_output=True)
+    return {v: ctypes.CDLL(str(ROOT / "_build" / "emul" / f"libccs_warp_{v}.so")) for v in ("full", "small", "tiny")}
+
+
+@pytest.mark.parametrize("name", KINDS)
+def test_probe_arithmetic_matches_oracle(libs, oracle, name):
+    oracle.set_kind(name)
+    words = oracle.unrank(np.random.default_rng(17).integers(0, oracle.n_entries(), 500, dtype=np.uint64))
+    out = np.zeros(len(words), np.uint64)
+    for m, left in [(-1, 0)] + [(m, left) for m in range(18) for left in (0, 1)]:
+        assert libs["full"].emul_warp_index(name.encode(), ctypes.c_void_p(words.ctypes.data), len(words), m, left,
+                                            ctypes.c_void_p(out.ctypes.data)) == 0
+        assert np.array_equal(out, oracle.index(words, -2 - m if left else m)), (m, left)
+
+
+def test_block_decode_of_every_entry(libs):
+    sectors = np.random.default_rng(3).integers(0, 1 << 32, (124, 8), dtype=np.uint64).astype(np.uint32)
+    entry, out = np.arange(124, dtype=np.uint32), np.zeros(124, np.uint32)
+    libs["full"].emul_warp_decode(ctypes.c_void_p(sectors.ctypes.data), ctypes.c_void_p(entry.ctypes.data), 124,
+                                  ctypes.c_void_p(out.ctypes.data))
+    b = np.unpackbits(sectors.view(np.uint8), axis=1, bitorder="little")
+    want = [int(sectors[j, 0] & 0xFF) + int(b[j, 8 + 2 * j]) + 2 * int(b[j, 9 + 2 * j]) for j in range(124)]
+    assert out.tolist() == want
+
+
+@pytest.mark.parametrize("size", ["full", "small", "tiny"])
+@pytest.mark.parametrize("name,starving", [("304", 0), ("s4", 1)])
+def test_every_node_is_searched_once(libs, size, name, starving):
+    """With all bounds zero nothing is pruned, so a completed iteration visits every canonical sequence
+    up to its bound (a prefix's moves once per item): the counts tell a lost or repeated node.  The
+    prefix lengths for bounds 1 to 4 are 1, 2, 3 and 4 moves, with donations 1, 1, 2 and 3."""
+
+    scrambles = [s[:4] for s in workloads.small_scrambles(2, seed=5)]
+    states = [workloads.scramble_state(s) for s in scrambles] + [CubieState()]
+    words, n = state_words(states), len(states)
+    lengths, moves = np.zeros(n, np.uint32), np.zeros((n, 24), np.uint8)
+    nodes, donated = np.zeros((n, 24), np.uint64), ctypes.c_uint64()
+    ptr = [ctypes.c_void_p(a.ctypes.data) for a in (words, lengths, moves, nodes)]
+    assert libs[size].emul_warp_solve(name.encode(), ptr[0], n, starving, ptr[1], ptr[2], ptr[3], ctypes.byref(donated)) == 0
+    count = [len(canonical_prefixes(L)) for L in range(5)]
+    full = {1: count[1], 2: 2 * count[2], 3: 3 * count[3]}
+    if starving:
+        full = {1: count[1], 2: count[1] + count[2], 3: 2 * count[2] + count[3]}
+    for s, length, mv, it in zip(states, lengths, moves, nodes):
+        assert length <= 4 and apply_moves(s, [MOVES_HTM[m] for m in mv[:length]]) == CubieState()
+        assert [int(it[b]) for b in range(1, length)] == [full[b] for b in range(1, length)]
+    assert lengths[-1] == 0 and max(lengths) == 4
+    assert not starving or donated.value > 0
