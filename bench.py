@@ -389,9 +389,9 @@ def reference_arm(args, world: int, rank: int, local: int) -> None:
 
 
 def bfs_roofline(passes: list[dict], entries: int, peak_gbs: float, ceiling: float | None) -> dict:
-    """The table build's passes against their rooflines: algorithmic bytes of a pass = one
-    sequential scan of the depth bytes (one per entry) + one 32-byte sector per random read and
-    per claim; the random sectors also against the random-sector ceiling."""
+    """The table build's passes against their rooflines: algorithmic bytes of a pass = a byte per
+    entry (its distance planes read and written) + the 32-byte sectors read at neighbours and claimed;
+    these also against the random-sector ceiling."""
 
     rows = []
     for p in passes:
@@ -409,11 +409,11 @@ def bfs_roofline(passes: list[dict], entries: int, peak_gbs: float, ceiling: flo
         out["achieved_gb_s"] = top["achieved_gb_s"]
         out["frac_of_hbm_peak"] = top["achieved_gb_s"] / peak_gbs
         if ceiling:
-            # Neighbours of nearby entries share classes, so most of a pass's random accesses hit
-            # L2: a rate above the DRAM random-sector ceiling says so, it is not a fraction of it.
+            # Neighbours come in whole blocks of frontier bits, many from L2: a rate above the DRAM
+            # random-sector ceiling says so, it is not a fraction of it.
             out["random_rate_over_dram_random_ceiling"] = top["random_sectors_per_s"] / ceiling
             out["note"] = ("random accesses costed as 32-byte sectors; a rate above the search's DRAM "
-                           "random-sector ceiling means most of them hit L2 (profiles/bfs_s4_dram.md: "
+                           "random-sector ceiling means most of them hit L2 (profiles/bfs_rows_304.md: "
                            "DRAM bytes per pass)")
     return out
 

@@ -1,15 +1,18 @@
 // libccs: building (BFS) and loading solving tables.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <chrono>
 #include <cstdarg>
 #include <cstdio>
 #include <cstddef>
 #include <cstring>
+#include <memory>
 #include <string>
 #include <vector>
 
-#include "bfs_kernel.cuh"
+#include "bfs_rows.cuh"
+#include "table_kernels.cuh"
 #include "ccs_internal.h"
 #include "dispatch.cuh"
 
@@ -232,163 +235,190 @@ static int build_impl(ccs_handle* h, const char* kind, const char* const paths[3
     CCS_TRY(set_kind(h, kind));
     CCS_CUDA_TRY(cudaSetDevice(h->device));
     const KindDesc k = h->kind;
-    const uint64_t n_entries = k.n_entries;
-    const uint64_t n_chunks = (n_entries + 15) / 16;
     auto t0 = std::chrono::steady_clock::now();
 
     // keep_resident 1: the new table replaces the handle's tables; 2: it becomes the second table.
     if (keep_resident == 2 && !h->d_table) return fail(CCS_E_STATE, "no first table to attach a second one to");
     if (keep_resident == 1) free_table(h);
-    DeviceBuffer<uint8_t> depth(n_chunks * 16);
-    DeviceBuffer<unsigned long long> counter(40);
-    if (!depth.ok() || !counter.ok())
-        return fail(CCS_E_NOMEM, "device allocation for the BFS (%llu bytes)", (unsigned long long)(n_chunks * 16));
-    CCS_CUDA_TRY(cudaMemsetAsync(depth.p, 0xFF, n_chunks * 16, h->stream));
-    CCS_CUDA_TRY(cudaMemsetAsync(counter.p, 0, 40 * sizeof(unsigned long long), h->stream));
-
-    BfsParams P;
-    P.depth = depth.p;
-    P.n_entries = n_entries;
-    P.n_chunks = n_chunks;
-    P.classidx = h->d_classidx;
-    P.class_rep = h->d_class_rep;
-    P.class_stab = h->d_class_stab;
-    P.counter = counter.p;
-    const int grid = h->sms * 8;
-
-    std::vector<uint64_t> counts;
-    auto read_counter = [&](uint64_t* v) -> int {
-        CCS_CUDA_TRY(cudaMemcpyAsync(v, counter.p, 8, cudaMemcpyDeviceToHost, h->stream));
-        CCS_CUDA_TRY(cudaStreamSynchronize(h->stream));
-        CCS_CUDA_TRY(cudaMemsetAsync(counter.p, 0, 8, h->stream));
-        return CCS_OK;
-    };
-    // per pass: entries found, random depth-byte reads, claim attempts, device time
-    h->last_passes.clear();
-    cudaEvent_t pe0, pe1;
-    CCS_CUDA_TRY(cudaEventCreate(&pe0));
-    CCS_CUDA_TRY(cudaEventCreate(&pe1));
-    struct EventPair {
-        cudaEvent_t a, b;
-        ~EventPair() { cudaEventDestroy(a); cudaEventDestroy(b); }
-    } ev_guard{pe0, pe1};
-    auto read_pass = [&](uint32_t d, bool fwd, uint64_t* found) -> int {
-        unsigned long long c[3];
-        CCS_CUDA_TRY(cudaMemcpyAsync(c, counter.p, sizeof c, cudaMemcpyDeviceToHost, h->stream));
-        CCS_CUDA_TRY(cudaStreamSynchronize(h->stream));
-        CCS_CUDA_TRY(cudaMemsetAsync(counter.p, 0, sizeof c, h->stream));
-        float ms = 0;
-        CCS_CUDA_TRY(cudaEventElapsedTime(&ms, pe0, pe1));
-        ccs_bfs_pass rec{};
-        rec.depth = (int32_t)d + 1;
-        rec.forward = fwd ? 1 : 0;
-        rec.found = c[0];
-        rec.random_reads = c[1];
-        rec.claims = c[2];
-        rec.seconds = ms * 1e-3;
-        h->last_passes.push_back(rec);
-        *found = c[0];
-        return CCS_OK;
-    };
-    CCS_TRY(dispatch_kind(k, [&](auto M, auto N) {
+    return dispatch_kind(k, [&](auto M, auto N) {
         constexpr int MODE = decltype(M)::value, NEC = decltype(N)::value;
-        bfs_seed<MODE, NEC><<<1, 32, 0, h->stream>>>(h->d_tables, P);
+        using RT = Rows<MODE, NEC>;
+        using Word = typename RT::Word;
+        const uint64_t n_entries = k.n_entries;
+        const uint64_t n_words = (n_entries + 15) / 16;
+        // A frontier of up to PUSH_MAX entries is a list, expanded forward; the one after it may hold 14
+        // times as many.  (Forward costs about 18 random claims an entry, a dense pass 5 ms and more:
+        // on d4t depths 1 to 7 take 0.9 ms in all as lists.)
+        constexpr uint32_t PUSH_MAX = 4u << 20;
+        DeviceBuffer<uint32_t> codes(RT::N_ROWS * RT::QW);
+        auto bits = std::make_unique<DeviceBuffer<Word>>(2 * RT::N_ROWS);
+        auto late = std::unique_ptr<DeviceBuffer<Word>>();
+        DeviceBuffer<uint8_t> flags(2 * RT::N_BLOCKS);
+        auto lists = std::make_unique<DeviceBuffer<uint64_t>>(2ull * PUSH_MAX);
+        DeviceBuffer<uint32_t> cmove(N_CLASSES * 18u), lut(RT::N_LUT * RT::LUT);
+        DeviceBuffer<uint4> desc(N_SLICE * 18u * 16u);
+        DeviceBuffer<unsigned long long> counter(4);
+        if (!codes.ok() || !bits->ok() || !flags.ok() || !lists->ok() || !cmove.ok() || !lut.ok() || !desc.ok() || !counter.ok())
+            return fail(CCS_E_NOMEM, "device allocation for the BFS (%llu bytes)",
+                        (unsigned long long)(RT::N_ROWS * (4u * RT::QW + 2u * sizeof(Word))));
+        CCS_CUDA_TRY(cudaMemsetAsync(codes.p, 0xFF, RT::N_ROWS * RT::QW * 4u, h->stream));
+        CCS_CUDA_TRY(cudaMemsetAsync(bits->p, 0, 2 * RT::N_ROWS * sizeof(Word), h->stream));
+        CCS_CUDA_TRY(cudaMemsetAsync(flags.p, 0, 2 * RT::N_BLOCKS, h->stream));
+        CCS_CUDA_TRY(cudaMemsetAsync(counter.p, 0, 4 * sizeof(unsigned long long), h->stream));
+
+        RowsParams P{};
+        P.codes = codes.p;
+        P.cur = bits->p, P.next = bits->p + RT::N_ROWS;
+        P.cur_flag = flags.p, P.next_flag = flags.p + RT::N_BLOCKS;
+        P.classidx = h->d_classidx;
+        P.class_rep = h->d_class_rep;
+        P.class_stab = h->d_class_stab;
+        P.cmove = cmove.p, P.desc = desc.p, P.lut = lut.p;
+        P.counter = counter.p;
+        rows_cmove<<<(N_CLASSES * 18u + 255u) / 256u, 256, 0, h->stream>>>(h->d_tables, P, cmove.p);
+        rows_desc<MODE><<<(N_SLICE * 18u * 16u + 255u) / 256u, 256, 0, h->stream>>>(h->d_tables, desc.p);
+        rows_lut<MODE, NEC><<<(RT::N_LUT * RT::LUT + 255u) / 256u, 256, 0, h->stream>>>(h->d_tables, lut.p);
         CCS_CUDA_TRY(cudaGetLastError());
-        uint64_t found = 0;
-        CCS_TRY(read_counter(&found));
-        counts.push_back(found);
-        uint64_t remaining = n_entries - found;
-        for (uint32_t d = 0; remaining; ++d) {
-            if (d >= 30) return fail(CCS_E_CHECK, "BFS deeper than 30");
-            // The reference's rule (table.py:112): forward while the frontier is under a
-            // quarter of the unvisited entries, backward afterwards.
-            bool forward = counts.back() < remaining / 4;
+
+        // per pass: entries found, random reads, claim attempts, device time
+        h->last_passes.clear();
+        cudaEvent_t pe0, pe1;
+        CCS_CUDA_TRY(cudaEventCreate(&pe0));
+        CCS_CUDA_TRY(cudaEventCreate(&pe1));
+        struct EventPair {
+            cudaEvent_t a, b;
+            ~EventPair() { cudaEventDestroy(a); cudaEventDestroy(b); }
+        } ev_guard{pe0, pe1};
+        unsigned long long c[4];
+        auto read_counters = [&]() -> int {
+            CCS_CUDA_TRY(cudaMemcpyAsync(c, counter.p, sizeof c, cudaMemcpyDeviceToHost, h->stream));
+            CCS_CUDA_TRY(cudaMemsetAsync(counter.p, 0, sizeof c, h->stream));
+            CCS_CUDA_TRY(cudaStreamSynchronize(h->stream));
+            return CCS_OK;
+        };
+        uint64_t *list = lists->p, *other = lists->p + PUSH_MAX;
+        rows_seed<MODE, NEC><<<1, 32, 0, h->stream>>>(h->d_tables, P, list, PUSH_MAX);
+        CCS_CUDA_TRY(cudaGetLastError());
+        CCS_TRY(read_counters());
+        std::vector<uint64_t> counts{c[0]};
+        uint64_t remaining = n_entries - c[0];
+        bool listed = true;
+        for (uint32_t d = 1; remaining; ++d) {  // d: the distance given in this pass
+            if (d > 30) return fail(CCS_E_CHECK, "BFS deeper than 30");
+            if (d == 15) {
+                late = std::make_unique<DeviceBuffer<Word>>(RT::N_ROWS);
+                if (!late->ok()) return fail(CCS_E_NOMEM, "device allocation for distances past 14");
+                rows_late<MODE, NEC><<<h->sms * 8, 256, 0, h->stream>>>(P, late->p);
+                P.late = reinterpret_cast<uint32_t*>(late->p);
+            }
             auto ts = std::chrono::steady_clock::now();
             CCS_CUDA_TRY(cudaEventRecord(pe0, h->stream));
-            if (forward) bfs_forward<MODE, NEC><<<grid, 256, 0, h->stream>>>(h->d_tables, P, d);
-            else bfs_backward<MODE, NEC><<<grid, 256, 0, h->stream>>>(h->d_tables, P, d);
+            const bool forward = listed;
+            if (forward) {
+                const uint32_t n = (uint32_t)counts.back();
+                const bool last = (uint64_t)n * 14u > PUSH_MAX || d >= 14;  // the next frontier as bits
+                rows_push<MODE, NEC><<<std::min<uint32_t>((n * 18u + 255u) / 256u, h->sms * 64), 256, 0, h->stream>>>(
+                    h->d_tables, P, list, n, last ? nullptr : other, PUSH_MAX, d);
+                std::swap(list, other);
+                listed = !last;
+            } else {
+                rows_pull<MODE, NEC><<<h->sms * 8, 256, 0, h->stream>>>(P, d);
+            }
             CCS_CUDA_TRY(cudaGetLastError());
             CCS_CUDA_TRY(cudaEventRecord(pe1, h->stream));
-            CCS_TRY(read_pass(d, forward, &found));
+            CCS_TRY(read_counters());
+            float ms = 0;
+            CCS_CUDA_TRY(cudaEventElapsedTime(&ms, pe0, pe1));
+            if (!listed) std::swap(P.cur, P.next), std::swap(P.cur_flag, P.next_flag);
+            ccs_bfs_pass rec{};
+            rec.depth = (int32_t)d;
+            rec.forward = forward ? 1 : 0;
+            rec.found = c[0];
+            rec.random_reads = c[1];
+            rec.claims = c[2];
+            rec.seconds = ms * 1e-3;
+            h->last_passes.push_back(rec);
             double dt = std::chrono::duration<double>(std::chrono::steady_clock::now() - ts).count();
-            log_msg(log, "depth %2u %s found %14llu (%7.2fs)", d + 1, forward ? "fwd" : "bwd", (unsigned long long)found, dt);
-            if (found == 0) return fail(CCS_E_UNREACHABLE, "%llu entries unreachable", (unsigned long long)remaining);
-            if (found > remaining) return fail(CCS_E_CHECK, "BFS found more entries than remain");
-            counts.push_back(found);
-            remaining -= found;
+            log_msg(log, "depth %2u %s found %14llu (%7.2fs)", d, forward ? "fwd" : "bwd", c[0], dt);
+            if (c[0] == 0) return fail(CCS_E_UNREACHABLE, "%llu entries unreachable", (unsigned long long)remaining);
+            if (c[0] > remaining) return fail(CCS_E_CHECK, "BFS found more entries than remain");
+            if (listed && c[3] != c[0]) return fail(CCS_E_CHECK, "BFS listed %llu of %llu entries", c[3], c[0]);
+            counts.push_back(c[0]);
+            remaining -= c[0];
         }
-        return CCS_OK;
-    }));
+        bits.reset();
+        lists.reset();
 
-    // Self-check: the histogram of depths equals the per-pass counts, nothing left unvisited.
-    {
-        DeviceBuffer<unsigned long long> hist(33);
-        if (!hist.ok()) return fail(CCS_E_NOMEM, "histogram buffer");
-        CCS_CUDA_TRY(cudaMemsetAsync(hist.p, 0, 33 * 8, h->stream));
-        bfs_histogram<<<h->sms * 4, 256, 0, h->stream>>>(depth.p, n_entries, hist.p);
-        CCS_CUDA_TRY(cudaGetLastError());
-        unsigned long long hh[33];
-        CCS_CUDA_TRY(cudaMemcpyAsync(hh, hist.p, sizeof hh, cudaMemcpyDeviceToHost, h->stream));
-        CCS_CUDA_TRY(cudaStreamSynchronize(h->stream));
-        for (int i = 0; i < 33; ++i) {
-            uint64_t want = i < (int)counts.size() ? counts[i] : 0;
-            if (hh[i] != want)
-                return fail(CCS_E_CHECK, "histogram of depth %d is %llu, BFS counted %llu", i, hh[i], (unsigned long long)want);
+        // Self-check: the histogram of depths equals the per-pass counts, nothing left unvisited.
+        {
+            DeviceBuffer<unsigned long long> hist(32);
+            if (!hist.ok()) return fail(CCS_E_NOMEM, "histogram buffer");
+            CCS_CUDA_TRY(cudaMemsetAsync(hist.p, 0, 32 * 8, h->stream));
+            rows_histogram<MODE, NEC><<<h->sms * 8, 256, 0, h->stream>>>(P, hist.p);
+            CCS_CUDA_TRY(cudaGetLastError());
+            unsigned long long hh[32];
+            CCS_CUDA_TRY(cudaMemcpyAsync(hh, hist.p, sizeof hh, cudaMemcpyDeviceToHost, h->stream));
+            CCS_CUDA_TRY(cudaStreamSynchronize(h->stream));
+            for (int i = 0; i < 32; ++i) {
+                uint64_t want = i < (int)counts.size() ? counts[i] : 0;
+                if (hh[i] != want)
+                    return fail(CCS_E_CHECK, "histogram of depth %d is %llu, BFS counted %llu", i, hh[i], (unsigned long long)want);
+            }
         }
-    }
 
-    // Encode: the block table always (the base-3 encoder reads its minima), the base-3 table when
-    // it is written or kept, then the mod-3 file; each file through "<path>.tmp" and a rename.
-    const uint64_t n_blk = (n_entries + BLOCK_ENTRIES - 1) / BLOCK_ENTRIES;
-    const uint64_t n_b3 = (n_entries + B3_ENTRIES - 1) / B3_ENTRIES;
-    DeviceBuffer<uint32_t> blk(n_blk * 8);
-    if (!blk.ok()) return fail(CCS_E_NOMEM, "block table allocation");
-    encode_block<<<h->sms * 8, 256, 0, h->stream>>>(depth.p, n_entries, n_blk, blk.p);
-    CCS_CUDA_TRY(cudaGetLastError());
-    const bool want_b3 = paths[CCS_FMT_B3] || (keep_resident && keep_format == CCS_FMT_B3);
-    DeviceBuffer<uint32_t> b3(want_b3 ? n_b3 * 8 : 0);
-    if (want_b3) {
-        if (!b3.ok()) return fail(CCS_E_NOMEM, "base-3 table allocation");
-        encode_b3<<<(unsigned)((n_b3 + 127) / 128), 128, 0, h->stream>>>(depth.p, blk.p, n_entries, n_b3, b3.p);
+        // Encode: the block table always (the base-3 encoder reads its minima), the base-3 table when
+        // it is written or kept, then the mod-3 file; each file through "<path>.tmp" and a rename.
+        const uint64_t n_blk = (n_entries + BLOCK_ENTRIES - 1) / BLOCK_ENTRIES;
+        const uint64_t n_b3 = (n_entries + B3_ENTRIES - 1) / B3_ENTRIES;
+        DeviceBuffer<uint32_t> blk(n_blk * 8);
+        if (!blk.ok()) return fail(CCS_E_NOMEM, "block table allocation");
+        encode_block<MODE, NEC><<<(unsigned)((n_blk + 255) / 256), 256, 0, h->stream>>>(P, n_entries, n_blk, blk.p);
         CCS_CUDA_TRY(cudaGetLastError());
-    }
-    cudaError_t e = cudaStreamSynchronize(h->stream);
-    if (e != cudaSuccess) return fail(CCS_E_CUDA, "encoding the table: %s", cudaGetErrorString(e));
-    double secs = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
-    if (seconds) *seconds = secs;
-    if (n_depths) *n_depths = (int)counts.size();
-    if (depth_counts)
-        for (int i = 0; i < (int)counts.size() && i < max_depths; ++i) depth_counts[i] = counts[i];
-
-    if (paths[CCS_FMT_MOD3]) {
-        DeviceBuffer<uint32_t> mod3(n_chunks);
-        if (!mod3.ok()) return fail(CCS_E_NOMEM, "mod-3 table allocation");
-        encode_mod3<<<h->sms * 8, 256, 0, h->stream>>>(depth.p, n_chunks, mod3.p);
-        CCS_CUDA_TRY(cudaGetLastError());
-        CCS_TRY(write_device_file(mod3.p, n_chunks * 4, paths[CCS_FMT_MOD3], h->stream));
-    }
-    if (paths[CCS_FMT_BLOCK]) CCS_TRY(write_device_file(blk.p, n_blk * 32, paths[CCS_FMT_BLOCK], h->stream));
-    if (paths[CCS_FMT_B3]) CCS_TRY(write_device_file(b3.p, n_b3 * 32, paths[CCS_FMT_B3], h->stream));
-
-    int rc = CCS_OK;
-    if (keep_resident == 1 || keep_resident == 2) {
-        DeviceBuffer<uint32_t>& kept = keep_format == CCS_FMT_B3 ? b3 : blk;
-        const uint64_t kept_bytes = keep_format == CCS_FMT_B3 ? n_b3 * 32 : n_blk * 32;
-        uint32_t* d_out = kept.release();
-        if (keep_resident == 1) {
-            free_table(h);
-            h->d_table = d_out;
-            h->table_bytes = kept_bytes;
-            h->format = keep_format;
-            restore.active = false;  // the new table is of the new kind
-        } else {
-            std::string second = h->kind_name;
-            rc = set_kind(h, first_kind.c_str());  // the constants stay those of the first table's kind
-            if (rc == CCS_OK) rc = attach_second(h, second.c_str(), keep_format, d_out, kept_bytes);
-            if (rc != CCS_OK) cudaFree(d_out);
+        const bool want_b3 = paths[CCS_FMT_B3] || (keep_resident && keep_format == CCS_FMT_B3);
+        DeviceBuffer<uint32_t> b3(want_b3 ? n_b3 * 8 : 0);
+        if (want_b3) {
+            if (!b3.ok()) return fail(CCS_E_NOMEM, "base-3 table allocation");
+            encode_b3<MODE, NEC><<<(unsigned)((n_b3 + 255) / 256), 256, 0, h->stream>>>(P, blk.p, n_entries, n_b3, b3.p);
+            CCS_CUDA_TRY(cudaGetLastError());
         }
-    }
-    return rc;
+        cudaError_t e = cudaStreamSynchronize(h->stream);
+        if (e != cudaSuccess) return fail(CCS_E_CUDA, "encoding the table: %s", cudaGetErrorString(e));
+        double secs = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+        if (seconds) *seconds = secs;
+        if (n_depths) *n_depths = (int)counts.size();
+        if (depth_counts)
+            for (int i = 0; i < (int)counts.size() && i < max_depths; ++i) depth_counts[i] = counts[i];
+
+        if (paths[CCS_FMT_MOD3]) {
+            DeviceBuffer<uint32_t> mod3(n_words);
+            if (!mod3.ok()) return fail(CCS_E_NOMEM, "mod-3 table allocation");
+            encode_mod3<MODE, NEC><<<(unsigned)((n_words + 255) / 256), 256, 0, h->stream>>>(P, n_entries, n_words, mod3.p);
+            CCS_CUDA_TRY(cudaGetLastError());
+            CCS_TRY(write_device_file(mod3.p, n_words * 4, paths[CCS_FMT_MOD3], h->stream));
+        }
+        if (paths[CCS_FMT_BLOCK]) CCS_TRY(write_device_file(blk.p, n_blk * 32, paths[CCS_FMT_BLOCK], h->stream));
+        if (paths[CCS_FMT_B3]) CCS_TRY(write_device_file(b3.p, n_b3 * 32, paths[CCS_FMT_B3], h->stream));
+
+        int rc = CCS_OK;
+        if (keep_resident == 1 || keep_resident == 2) {
+            DeviceBuffer<uint32_t>& kept = keep_format == CCS_FMT_B3 ? b3 : blk;
+            const uint64_t kept_bytes = keep_format == CCS_FMT_B3 ? n_b3 * 32 : n_blk * 32;
+            uint32_t* d_out = kept.release();
+            if (keep_resident == 1) {
+                free_table(h);
+                h->d_table = d_out;
+                h->table_bytes = kept_bytes;
+                h->format = keep_format;
+                restore.active = false;  // the new table is of the new kind
+            } else {
+                std::string second = h->kind_name;
+                rc = set_kind(h, first_kind.c_str());  // the constants stay those of the first table's kind
+                if (rc == CCS_OK) rc = attach_second(h, second.c_str(), keep_format, d_out, kept_bytes);
+                if (rc != CCS_OK) cudaFree(d_out);
+            }
+        }
+        return rc;
+    });
 }
 
 extern "C" int ccs_build_table(ccs_handle* h, const char* kind, int format, const char* out_path, int keep_resident,

@@ -211,8 +211,10 @@ class Preset:
 
     @property
     def build_bytes(self) -> int:
-        """Peak device memory of building it here: one exact-depth byte per entry (padded to 16)
-        and the encoded block table, plus the base-3 table while it is encoded from the block one."""
+        """Device memory that building it here asks for: a byte per entry (padded to 16) and the encoded
+        block table, plus the base-3 table while it is encoded from the block one.  (The build stays
+        within it: six or, past depth 14, seven bits' planes per entry while it searches, four or five
+        beside the tables.)"""
 
         depth = -(-self.entries // 16) * 16
         block = -(-self.entries // BLOCK_ENTRIES) * 32

@@ -115,11 +115,11 @@ int ccs_save_table(ccs_handle* h, int table, const char* path);
  * and "at least" at the cut of either format).  The bins sum to the kind's entry count. */
 int ccs_table_histogram(ccs_handle* h, int table, uint64_t* bins, int n_bins);
 
-/* One BFS pass of the last ccs_build_table: the depth it assigned, forward (1: expand the
- * frontier, kernels.cu:544-574) or backward (0: unvisited entries test their neighbours,
- * kernels.cu:577-611), the entries found, the random depth-byte reads and the claim attempts
- * (atomics) it made, and its device time.  Algorithmic bytes of a pass: one sequential scan of
- * the depth bytes plus one 32-byte sector per random read and per claim. */
+/* One BFS pass of the last ccs_build_table: the depth it assigned, forward (1: expand the listed
+ * frontier, kernels.cu:544-574) or backward (0: unvisited entries look for a neighbour in the
+ * frontier, kernels.cu:577-611), the entries found, the 32-byte sectors read at neighbours (one per
+ * neighbour forward, whole blocks of frontier bits backward) and the claim attempts (atomics, forward
+ * only) it made, and its device time. */
 typedef struct ccs_bfs_pass {
     int32_t depth;
     int32_t forward;
