@@ -100,13 +100,24 @@ __device__ __forceinline__ uint32_t warp_edge_coord(const WarpTables& T, const S
     }
 }
 
+// The same bound as decode_sector.  The word is found in three halvings.  A base-3 digit k of a byte is
+// the integer part of 3 x the fraction of byte / 3^(k + 1), that fraction being byte * 3^(4 - k) times
+// 1/243 as a 32-bit fraction (rounded up: off by less than 2^-17, digits are 1/243 apart): two
+// multiplies where a division by a power chosen at run time took a loop of them.
 template <int FMT>
 __device__ __forceinline__ uint32_t warp_decode(const uint32_t w[8], uint32_t j) {
-    if (FMT == FMT_B3) return decode_sector<FMT_B3>(w, j);
-    const uint32_t q = (j + 4u) >> 4;  // word of the offset, found in three halvings
+    const uint32_t q5 = j / 5u;                                           // (base 3: byte 1 + q5, digit j % 5)
+    const uint32_t q = FMT == FMT_B3 ? (q5 + 1u) >> 2 : (j + 4u) >> 4;    // word
     const bool b0 = q & 1u, b1 = q & 2u, b2 = q & 4u;
     const uint32_t a = b0 ? w[1] : w[0], b = b0 ? w[3] : w[2], c = b0 ? w[5] : w[4], d = b0 ? w[7] : w[6];
     const uint32_t e = b1 ? b : a, f = b1 ? d : c, v = b2 ? f : e;
+    if (FMT == FMT_B3) {
+        const uint32_t byte = (v >> ((8u * q5 + 8u) & 31u)) & 0xFFu;
+        const uint32_t power = prmt_raw(0x03091B51u, 1u, (j - 5u * q5) | 0x7770u);  // 81, 27, 9, 3, 1
+        const uint32_t digit = (uint32_t)(((unsigned long long)(byte * power * 17674763u) * 3u) >> 32);
+        const uint32_t m = w[0] & 63u;
+        return digit ? m + ((w[0] >> 6) & 3u) + digit : m;
+    }
     return (w[0] & 0xFFu) + ((v >> ((2u * j + 8u) & 31u)) & 3u);
 }
 

@@ -188,6 +188,10 @@ void emul_warp_decode(const uint32_t* sectors, const uint32_t* entry, int n, uin
     for (int i = 0; i < n; ++i) out[i] = warp_decode<FMT_BLOCK>(sectors + 8 * i, entry[i]);
 }
 
+void emul_warp_decode_b3(const uint32_t* sectors, const uint32_t* entry, int n, uint32_t* out) {
+    for (int i = 0; i < n; ++i) out[i] = warp_decode<FMT_B3>(sectors + 8 * i, entry[i]);
+}
+
 // Solves n cubes (at most 8) with one warp on an all-zero table; `starving`: with shorter
 // prefixes, donating all the time.  lengths[n]; nodes[24 n]: per cube and bound.  Returns the error bits (-1: unfinished).
 int emul_warp_solve(const char* name, const uint32_t* words, int n, int starving, uint32_t* lengths, uint8_t* moves,

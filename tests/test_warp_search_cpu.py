@@ -46,6 +46,19 @@ def test_block_decode_of_every_entry(libs):
     assert out.tolist() == want
 
 
+def test_base3_decode_of_every_byte_and_entry(libs):
+    """Every value of a byte at every one of the 155 entries, against digits by division."""
+
+    byte, entry = (a.ravel() for a in np.meshgrid(np.arange(256), np.arange(155), indexing="ij"))
+    sectors = np.random.default_rng(4).integers(0, 256, (len(entry), 32), dtype=np.uint8)
+    sectors[np.arange(len(entry)), 1 + entry // 5] = byte
+    words, at, out = sectors.view(np.uint32).copy(), entry.astype(np.uint32), np.zeros(len(entry), np.uint32)
+    libs["full"].emul_warp_decode_b3(*(ctypes.c_void_p(a.ctypes.data) for a in (words, at)), len(at), ctypes.c_void_p(out.ctypes.data))
+    head = sectors[:, 0].astype(np.int64)
+    digit = byte // 3 ** (entry % 5) % 3
+    assert np.array_equal(out, (head & 63) + np.where(digit == 0, 0, (head >> 6) + digit))
+
+
 @pytest.mark.parametrize("size", ["full", "small", "tiny"])
 @pytest.mark.parametrize("name,starving", [("304", 0), ("s4", 1)])
 def test_every_node_is_searched_once(libs, size, name, starving):
