@@ -98,7 +98,10 @@ void fill_params(ccs_handle* h, const ccs_solve_opts* o, SearchParams* P) {
     // keeps a warp busy past the walk to it, and 2,960 warps need some items each.  With many cubes
     // in flight other cubes fill the warps, and longer items cost fewer walks.
     P->warp_items = resolve_variant(o, 0) == 12 ? 1u : 0u;
-    P->warp_at[0] = 20000ull;
+    // (1,500: a lone cube's iteration after one of 3,400 nodes took 250 us with 243 items -- most warps had
+    // none and the largest item was a long chain -- and 147 us with 3,240.  The second threshold stays: at
+    // 60,000 the iteration after the next took 470 us against 410, 43,239 items being too many for it.)
+    P->warp_at[0] = 1500ull;
     P->warp_at[1] = 200000ull;
     P->warp_many_at[0] = 300000ull;
     P->warp_many_at[1] = 30000000ull;
