@@ -252,20 +252,50 @@ def flipped_edges(words: np.ndarray) -> np.ndarray:
     return ((b[:, 8:] >> 4) & 1).sum(axis=1)
 
 
+def _move_steps() -> tuple[np.ndarray, np.ndarray]:
+    """Per move (18: none), the byte of a packed state that each of its 20 bytes comes from, and what
+    that byte becomes (by its value)."""
+
+    src, becomes = np.empty((19, 20), np.int64), np.empty((19, 20, 256), np.uint8)
+    values = np.arange(256, dtype=np.uint8)
+    src[18], becomes[18] = np.arange(20), values
+    for m, move in enumerate(MOVES_HTM):
+        src[m] = list(move.cp) + [8 + p for p in move.ep]
+        for i in range(8):
+            becomes[m, i] = (values & 7) | (((values >> 3) + move.co[i]) % 3 << 3)
+        for i in range(12):
+            becomes[m, 8 + i] = values ^ (move.eo[i] << 4)
+    return src, becomes
+
+
+_SRC, _BECOMES = _move_steps()
+_STEPS = [[(int(_SRC[m, i]), _BECOMES[m, i].tobytes()) for i in range(20)] for m in range(18)]
+_SOLVED = list(range(8)) + list(range(12))
+# Up to this many cubes are checked one by one in plain Python (14 us each at 18 moves), more of them a
+# column of moves at a time (0.19 ms for 13 cubes, 0.6 for 100; before, by distinct moves, 0.3 for one).
+_CHECK_ONE_BY_ONE = 12
+
+
 def verify_solutions(words: np.ndarray, solutions: list[list[int]]) -> bool:
     """True if every move list takes its packed state (n, 5) to solved (the reference's host
-    self-check, solver.py:317-319, vectorised over cubes)."""
+    self-check, solver.py:317-319).  Negative entries are no moves."""
 
     b = np.ascontiguousarray(words, np.uint32).reshape(-1, 5).view(np.uint8).reshape(-1, 20)
-    corners, edges = b[:, :8].copy(), b[:, 8:].copy()
-    longest = max((len(m) for m in solutions), default=0)
-    for j in range(longest):
-        col = np.array([m[j] if j < len(m) else -1 for m in solutions])
-        for mv in np.unique(col[col >= 0]):
-            rows = col == mv
-            corners[rows], edges[rows] = coords.apply_move(corners[rows], edges[rows], int(mv))
-    solved = np.concatenate([np.arange(8, dtype=np.uint8)[None], np.arange(12, dtype=np.uint8)[None]], axis=1)
-    return bool((np.concatenate([corners, edges], axis=1) == solved).all())
+    if len(b) <= _CHECK_ONE_BY_ONE and len(b) == len(solutions):
+        for state, moves in zip(b.tolist(), solutions):
+            for m in moves:
+                if m >= 0:
+                    state = [becomes[state[src]] for src, becomes in _STEPS[m]]
+            if state != _SOLVED:
+                return False
+        return True
+    if any(m > 17 for moves in solutions for m in moves):
+        raise IndexError("a move is 0 to 17")
+    at = np.arange(20)
+    for j in range(max((len(m) for m in solutions), default=0)):
+        col = np.array([m[j] if j < len(m) and m[j] >= 0 else 18 for m in solutions])
+        b = _BECOMES[col[:, None], at, np.take_along_axis(b, _SRC[col], axis=1)]
+    return bool((b == _SOLVED).all())
 
 
 def parse_moves(text: str) -> list[int]:
