@@ -556,7 +556,18 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_warp(const WarpTa
                     dry = false;
                     build = 2;
                 }
-                if (found) build = 0, dry = true;  // solved by another unit: this one only counts as done
+                if (found) {  // solved by another unit: this one only counts as done ...
+                    build = 0;
+                    dry = true;
+                    if (r == FETCH_OK) {  // ... and with it all items not handed out yet, up to 10 M of them
+                        // (the iteration cannot end meanwhile, so its ticket is the one that was drawn from)
+                        const uint32_t items = P.n_prefix[plen];
+                        uint32_t next = items;
+                        if (lane == 0) next = (uint32_t)atomicMax(&P.slots[slot].ticket, ticket_make(plen, bound, epoch) | items);
+                        next = __shfl_sync(FULL, next, 0);
+                        held += next < items ? items - next : 0u;
+                    }
+                }
             }
             if (build) {
                 const uint32_t at = __ffs(free_places()) - 1u;

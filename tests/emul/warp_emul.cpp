@@ -124,6 +124,7 @@ static void __threadfence_system() {}
 template <class T, class U> static T atomicAdd(T* p, U v) { T o = *p; *p = o + (T)v; return o; }
 template <class T, class U> static T atomicSub(T* p, U v) { T o = *p; *p = o - (T)v; return o; }
 template <class T, class U> static T atomicExch(T* p, U v) { T o = *p; *p = (T)v; return o; }
+template <class T, class U> static T atomicMax(T* p, U v) { T o = *p; if ((T)v > o) *p = (T)v; return o; }
 template <class T, class U> static T atomicOr(T* p, U v) { T o = *p; *p = o | (T)v; return o; }
 template <class T, class U, class V> static T atomicCAS(T* p, U c, V v) { T o = *p; if (o == (T)c) *p = (T)v; return o; }
 
@@ -191,6 +192,9 @@ void emul_warp_decode(const uint32_t* sectors, const uint32_t* entry, int n, uin
 void emul_warp_decode_b3(const uint32_t* sectors, const uint32_t* entry, int n, uint32_t* out) {
     for (int i = 0; i < n; ++i) out[i] = warp_decode<FMT_B3>(sectors + 8 * i, entry[i]);
 }
+
+// Warp intrinsics that the last emul_warp_solve ran: its length in steps of the warp.
+uint64_t emul_warp_turns() { return arrived[0]; }
 
 // Solves n cubes (at most 8) with one warp on an all-zero table; `starving`: with shorter
 // prefixes, donating all the time.  lengths[n]; nodes[24 n]: per cube and bound.  Returns the error bits (-1: unfinished).

@@ -82,3 +82,17 @@ def test_every_node_is_searched_once(libs, size, name, starving):
         assert [int(it[b]) for b in range(1, length)] == [full[b] for b in range(1, length)]
     assert lengths[-1] == 0 and max(lengths) == 4
     assert not starving or donated.value > 0
+
+
+def test_items_of_a_solved_cube_are_dropped_together(libs):
+    """The iteration that finds a cube's solution hands out up to millions of items; the ones left are counted
+    as done at once, not fetched one by one (43,254 of them here; a fetch is some 35 of the warp's steps)."""
+
+    back = [0, 4, 8, 9, 13]  # (an early one of the items)
+    state = apply_moves(CubieState(), [MOVES_HTM[3 * (m // 3) + 2 - m % 3] for m in reversed(back)])
+    words, length, moves = state_words([state]), np.zeros(1, np.uint32), np.zeros(24, np.uint8)
+    nodes, donated = np.zeros(24, np.uint64), ctypes.c_uint64()
+    ptr = [ctypes.c_void_p(a.ctypes.data) for a in (words, length, moves, nodes)]
+    assert libs["full"].emul_warp_solve(b"s4", ptr[0], 1, 0, ptr[1], ptr[2], ptr[3], ctypes.byref(donated)) == 0
+    libs["full"].emul_warp_turns.restype = ctypes.c_uint64
+    assert length[0] == 5 and libs["full"].emul_warp_turns() < 20 * len(canonical_prefixes(4))
