@@ -146,6 +146,11 @@ int set_kind(ccs_handle* h, const char* name) {
     }
     auto T = std::make_unique<DevImage>();
     build_dev_tables(k, &T->t);
+    if (h->d_table2) {  // the second table's E-content classes go with every image
+        KindDesc k2;
+        TRY(get_kind(h->kind2_name.c_str(), &k2));
+        build_genc(k2, T->t.genc2);
+    }
     build_warp_tables(T->t, &T->w);
     CUDA_TRY(cudaMemcpy(h->d_image, T.get(), sizeof(DevImage), cudaMemcpyHostToDevice));
     h->kind = k;

@@ -93,3 +93,16 @@ def test_table_id_errors(dual):
     lone = resident_handle("d4t")
     with pytest.raises(native.CcsError, match="second table"):
         lone.solve(words, None, np.array([1], np.uint8))
+
+
+def test_building_another_kind_keeps_the_second_table(dual, lengths_golden):
+    """A build that keeps nothing takes the handle's constants through another kind and back; the second
+    table's own class map has to come back with them."""
+
+    words = state_words(_states(lengths_golden["random1000"][4:10]))
+    opts, ids = native.solve_opts(timeout_s=300), np.ones(6, np.uint8)
+    before = dual.solve(words, opts, ids)
+    dual.build_table("304", "block", None, keep_resident=0)
+    for a, b in zip(before, dual.solve(words, opts, ids)):
+        assert a.length == b.length
+        assert list(a.iter_nodes[: a.length]) == list(b.iter_nodes[: b.length])
