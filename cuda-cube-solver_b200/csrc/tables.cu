@@ -122,8 +122,11 @@ int read_file_to_device(FILE* f, void* d, uint64_t n_bytes, const char* path, cu
 extern "C" int ccs_load_table(ccs_handle* h, const char* kind, int format, const char* path) {
     if (!h || !kind || !path) return fail(CCS_E_ARG, "NULL argument");
     if (format != CCS_FMT_BLOCK && format != CCS_FMT_B3) return fail(CCS_E_ARG, "unknown table format %d", format);
-    CCS_TRY(set_kind(h, kind));
-    uint64_t want = table_bytes_for(h->kind, format);
+    KindDesc k;
+    CCS_TRY(get_kind(kind, &k));
+    if (!kind_supported(k)) return fail(CCS_E_ARG, "kind %s: %d E-content classes are not compiled in", kind, k.nec);
+    if (!h->d_table) CCS_TRY(set_kind(h, kind));  // (a resident table's kind stays until the file has been checked)
+    uint64_t want = table_bytes_for(k, format);
     FILE* f = fopen(path, "rb");
     if (!f) return fail(CCS_E_FILE, "%s not found", path);
     fseek(f, 0, SEEK_END);
@@ -135,6 +138,10 @@ extern "C" int ccs_load_table(ccs_handle* h, const char* kind, int format, const
     }
     CCS_CUDA_TRY(cudaSetDevice(h->device));
     free_table(h);
+    if (const int rc = set_kind(h, kind); rc != CCS_OK) {
+        fclose(f);
+        return rc;
+    }
     uint32_t* d = nullptr;
     if (cudaMalloc(&d, want) != cudaSuccess) {
         fclose(f);

@@ -254,3 +254,18 @@ def test_building_another_kind_leaves_the_resident_table_usable(tmp_path):
         assert h.lower_bound(words).tolist() == before
     finally:
         h.close()
+
+
+def test_refused_load_keeps_the_resident_kind(tmp_path):
+    """A load of another kind that is refused (no such file, a wrong size) leaves the handle on the kind of
+    its resident table: searches would otherwise index that table as the other kind."""
+
+    h = resident_handle("d4t")
+    words = state_words([apply_moves(CubieState(), [MOVES_HTM[m] for m in (0, 4, 8, 9, 13)])])
+    want = h.index(words)[0].tolist()
+    short = tmp_path / "short.bin"
+    short.write_bytes(b"\0" * 64)
+    for path in (tmp_path / "missing.bin", short):
+        with pytest.raises(native.CcsError):
+            h.load_table("304", "block", path)
+        assert h.index(words)[0].tolist() == want
