@@ -263,6 +263,21 @@ __global__ void __launch_bounds__(256) rows_push(const DevTables* __restrict__ g
     add_count(P.counter + 2, claims);
 }
 
+// The frontier bits of distance d (at most 14), read off the planes: for a frontier that outgrew its list,
+// whose claims past the list's end were given their distance but not listed.
+template <int MODE, int NEC>
+__global__ void __launch_bounds__(256) rows_mark(RowsParams P, uint64_t n_rows, uint32_t d) {
+    using RT = Rows<MODE, NEC>;
+    for (uint64_t row = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; row < n_rows; row += (uint64_t)gridDim.x * blockDim.x) {
+        uint32_t p[4], eq = RT::ALL;
+        load_codes<RT>(P.codes, row, p);
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) eq &= (d >> j) & 1u ? p[j] : ~p[j];
+        reinterpret_cast<typename RT::Word*>(P.next)[row] = (typename RT::Word)eq;
+        if (eq) P.next_flag[row / RT::R] = 1u;
+    }
+}
+
 // ---- dense passes: unreached entries look for a neighbour in the frontier --------------------------
 
 // The lane's k-th row of a block.  Group kinds: rows k = 0..3 have even flip parity, 4..7 odd, so

@@ -136,6 +136,27 @@ void encode(const uint8_t* dist, uint64_t n, int late, uint32_t* blk, uint32_t* 
     for (thread_no = 0; thread_no < nm; ++thread_no) encode_mod3<MODE, NEC>(P, n, nm, mod3);
 }
 
+// Frontier bits of distance d on given distances, of whole rows (n: a multiple of the kind's columns), and the
+// flags of their blocks.
+template <int MODE, int NEC>
+void mark(const uint8_t* dist, uint64_t n, uint32_t d, uint8_t* bits, uint8_t* flags) {
+    using RT = Rows<MODE, NEC>;
+    const uint64_t rows = n / RT::C;
+    std::vector<uint32_t> codes(rows * RT::QW, ~0u);
+    std::vector<typename RT::Word> next(rows, 0);
+    for (uint64_t i = 0; i < n; ++i) {
+        uint32_t p[4];
+        load_codes<RT>(codes.data(), i / RT::C, p);
+        for (int b = 0; b < 4; ++b)
+            if (!((dist[i] >> b) & 1u)) p[b] &= ~(1u << (i % RT::C));
+        store_codes<RT>(codes.data(), i / RT::C, p);
+    }
+    RowsParams P{};
+    P.codes = codes.data(), P.next = next.data(), P.next_flag = flags;
+    for (thread_no = 0; thread_no < 256u; ++thread_no) rows_mark<MODE, NEC>(P, rows, d);
+    for (uint64_t i = 0; i < n; ++i) bits[i] = (uint8_t)((next[i / RT::C] >> (i % RT::C)) & 1u);
+}
+
 template <typename F>
 int with_kind(const char* name, F&& f) {
     using std::integral_constant;
@@ -160,6 +181,11 @@ int emul_rows_neighbours(const char* name, const uint64_t* idx, int n, int m, ui
     static std::map<std::string, Structure> memo;
     return with_kind(name, [&](auto M, auto N, const DevTables& T) {
         neighbours<decltype(M)::value, decltype(N)::value>(T, idx, n, m, out, memo, name);
+    });
+}
+int emul_rows_mark(const char* name, const uint8_t* dist, uint64_t n, uint32_t d, uint8_t* bits, uint8_t* flags) {
+    return with_kind(name, [&](auto M, auto N, const DevTables&) {
+        mark<decltype(M)::value, decltype(N)::value>(dist, n, d, bits, flags);
     });
 }
 int emul_rows_encode(const char* name, const uint8_t* dist, uint64_t n, int late, uint32_t* blk, uint32_t* b3, uint32_t* mod3) {

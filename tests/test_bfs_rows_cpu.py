@@ -75,3 +75,17 @@ def test_encoders(rows, name, n, top):
     assert np.array_equal(b3, _b3(d))
     r = np.concatenate([d % 3, np.full(-n % 16, 3)]).reshape(-1, 16).astype(np.uint64)
     assert np.array_equal(mod3, (r << (2 * np.arange(16, dtype=np.uint64))).sum(axis=1).astype(np.uint32))
+
+
+@pytest.mark.parametrize("name,columns,block_rows", [("304", 16, 70), ("s4", 8, 256), ("d4f", 12, 256), ("a4t", 16, 256), ("d4t", 24, 256)])
+@pytest.mark.parametrize("d", [0, 7, 13])
+def test_frontier_read_off_the_planes(rows, name, columns, block_rows, d):
+    """The frontier of a pass that claimed more entries than its list holds: the bits of every entry of that
+    distance, and the flags of the blocks that have one."""
+
+    per_block = columns * block_rows
+    dist = np.random.default_rng(d).integers(0, 16, 3 * per_block).astype(np.uint8)
+    dist[per_block: 2 * per_block][dist[per_block: 2 * per_block] == d] = 15  # a block without any
+    bits, flags = np.zeros(len(dist), np.uint8), np.zeros(3, np.uint8)
+    assert rows.emul_rows_mark(name.encode(), _ptr(dist), ctypes.c_uint64(len(dist)), d, _ptr(bits), _ptr(flags)) == 0
+    assert np.array_equal(bits, dist == d) and flags.tolist() == [1, 0, 1]
