@@ -278,22 +278,27 @@ _CHECK_ONE_BY_ONE = 12
 
 def verify_solutions(words: np.ndarray, solutions: list[list[int]]) -> bool:
     """True if every move list takes its packed state (n, 5) to solved (the reference's host
-    self-check, solver.py:317-319).  Negative entries are no moves."""
+    self-check, solver.py:317-319).  Negative entries are no moves; a move above 17, or moves for another
+    number of cubes, raise IndexError."""
 
     b = np.ascontiguousarray(words, np.uint32).reshape(-1, 5).view(np.uint8).reshape(-1, 20)
-    if len(b) <= _CHECK_ONE_BY_ONE and len(b) == len(solutions):
+    if any(max(moves) >= 18 for moves in solutions if len(moves)):
+        raise IndexError("a move is 0 to 17")
+    if len(b) != len(solutions):
+        if any(max(moves) >= 0 for moves in solutions if len(moves)):
+            raise IndexError(f"moves for {len(solutions)} cubes, {len(b)} states")
+        return bool((b == _SOLVED).all())
+    if len(b) <= _CHECK_ONE_BY_ONE:
         for state, moves in zip(b.tolist(), solutions):
             for m in moves:
                 if m >= 0:
-                    state = [becomes[state[src]] for src, becomes in _STEPS[m]]
+                    state = [becomes[state[src]] for src, becomes in _STEPS[int(m)]]
             if state != _SOLVED:
                 return False
         return True
-    if any(m > 17 for moves in solutions for m in moves):
-        raise IndexError("a move is 0 to 17")
     at = np.arange(20)
     for j in range(max((len(m) for m in solutions), default=0)):
-        col = np.array([m[j] if j < len(m) and m[j] >= 0 else 18 for m in solutions])
+        col = np.array([int(m[j]) if j < len(m) and m[j] >= 0 else 18 for m in solutions])
         b = _BECOMES[col[:, None], at, np.take_along_axis(b, _SRC[col], axis=1)]
     return bool((b == _SOLVED).all())
 

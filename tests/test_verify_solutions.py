@@ -27,3 +27,16 @@ def test_right_and_wrong_solutions(n):
     assert not verify_solutions(state_words(workloads.uniform_cubes(n, seed=n)), [[] for _ in range(n)])
     with pytest.raises(IndexError):
         verify_solutions(words, back[:at] + [back[at] + [18]] + back[at + 1:])
+
+
+@pytest.mark.parametrize("n", [1, 12, 13, 60])
+def test_moves_for_another_number_of_cubes_are_refused(n):
+    words = state_words([apply_moves(CubieState(), [MOVES_HTM[0]])] * n)
+    assert verify_solutions(words, [[2]] * n)
+    for other in {1, n - 1, n + 1} - {n, 0}:
+        with pytest.raises(IndexError):
+            verify_solutions(words, [[2]] * other)
+    # a wrong move is refused wherever it stands, and moves may be any kind of number
+    with pytest.raises(IndexError):
+        verify_solutions(words, [[0]] * (n - 1) + [[0, 18]])
+    assert verify_solutions(words, [[2.0]] * n)
