@@ -298,7 +298,7 @@ def verify_solutions(words: np.ndarray, solutions: list[list[int]]) -> bool:
         return True
     at = np.arange(20)
     for j in range(max((len(m) for m in solutions), default=0)):
-        col = np.array([int(m[j]) if j < len(m) and m[j] >= 0 else 18 for m in solutions])
+        col = np.array([m[j] if j < len(m) and m[j] >= 0 else 18 for m in solutions]).astype(np.int64)
         b = _BECOMES[col[:, None], at, np.take_along_axis(b, _SRC[col], axis=1)]
     return bool((b == _SOLVED).all())
 
