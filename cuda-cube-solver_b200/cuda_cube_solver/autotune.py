@@ -43,6 +43,8 @@ SPACE = {
     "probe_min": [12, 16, 20, 24],
 }
 DEFAULT = {"variant": 12, "base_plen": 4, "move": (8, 4), "steal_depth": 2, "spread": 4096, "probe_min": 16}
+# Settings are kept with the search kernels they were measured on; those of other kernels are not used.
+KERNELS = "warp"
 MIN_GAIN = 0.02  # a setting must cut the sample's device time by 2% to replace the incumbent
 
 
@@ -111,7 +113,7 @@ def gpu_name(device: int = 0) -> str:
 def save(result: dict, table: str, n: int, device: int = 0) -> None:
     CACHE.parent.mkdir(parents=True, exist_ok=True)
     data = json.loads(CACHE.read_text()) if CACHE.exists() else {}
-    data[_key(gpu_name(device), table, n)] = result
+    data[_key(gpu_name(device), table, n)] = dict(result, kernels=KERNELS)
     CACHE.write_text(json.dumps(data, indent=1) + "\n")
 
 
@@ -119,7 +121,8 @@ def lookup(table: str, n: int, device: int = 0) -> dict | None:
     if not CACHE.exists():
         return None
     cfg = json.loads(CACHE.read_text()).get(_key(gpu_name(device), table, n))
-    if cfg:
-        cfg = dict(cfg["config"])
-        cfg["move"] = tuple(cfg["move"])
+    if not cfg or cfg.get("kernels") != KERNELS:
+        return None
+    cfg = dict(cfg["config"])
+    cfg["move"] = tuple(cfg["move"])
     return cfg

@@ -76,6 +76,20 @@ def test_autotune_cache_round_trip(tmp_path, monkeypatch):
     assert [autotune.batch_bucket(n) for n in (1, 10, 100, 5000)] == ["1", "small", "medium", "large"]
 
 
+def test_settings_of_other_kernels_are_not_used(tmp_path, monkeypatch):
+    """A cache entry without the kernels' name (written before the warp kernel) or with another one would
+    pick that kernel's variant over the default."""
+
+    monkeypatch.setattr(autotune, "CACHE", tmp_path / "cache.json")
+    result = {"config": dict(FakeHandle.BEST, variant=3, move=[8, 4]), "cubes_per_s": 1.0}
+    autotune.save(result, "d4t", 1000)
+    data = json.loads(autotune.CACHE.read_text())
+    assert autotune.lookup("d4t", 1000)["variant"] == 3
+    for other in ({}, {"kernels": "lane"}):
+        autotune.CACHE.write_text(json.dumps({k: result | other for k in data}))
+        assert autotune.lookup("d4t", 1000) is None
+
+
 class FakeServer:
     """Finishes request i after a fixed device latency of (i % 3 + 1) ms of host time."""
 
