@@ -45,6 +45,7 @@ SPACE = {
 DEFAULT = {"variant": 12, "base_plen": 4, "move": (8, 4), "steal_depth": 2, "spread": 4096, "probe_min": 16}
 # Settings are kept with the search kernels they were measured on; those of other kernels are not used.
 KERNELS = "warp"
+LANE_KNOBS = ("move", "probe_min")  # the warp kernel (variant 12) does not read them
 MIN_GAIN = 0.02  # a setting must cut the sample's device time by 2% to replace the incumbent
 
 
@@ -82,6 +83,8 @@ def tune(handle: native.Handle, states, table: str, rounds: int = 2, log=None, b
     out_of_time = False
     for _ in range(rounds):
         for knob, values in SPACE.items():
+            if best["variant"] == 12 and knob in LANE_KNOBS:
+                continue
             for v in values:
                 if v == best[knob]:
                     continue

@@ -54,6 +54,18 @@ def test_autotune_ignores_gains_within_noise():
     assert result["config"] == autotune.DEFAULT
 
 
+def test_autotune_skips_knobs_that_the_warp_kernel_ignores():
+    """With variant 12 the lane kernels' knobs change nothing: trying them could only pick noise."""
+
+    class Warp(FakeHandle):
+        BEST = dict(FakeHandle.BEST, variant=12, move=(16, 8), probe_min=24)
+
+    h = Warp()
+    config = autotune.tune(h, workloads.uniform_cubes(4, seed=9), "d4t", rounds=2)["config"]
+    assert config == dict(Warp.BEST, move=autotune.DEFAULT["move"], probe_min=autotune.DEFAULT["probe_min"])
+    assert {(o.move_min, o.move_age, o.probe_min) for o in h.calls if o.variant == 12} == {(8, 4, 16)}
+
+
 def test_autotune_stops_at_its_budget():
     h = FakeHandle()
     result = autotune.tune(h, workloads.uniform_cubes(4, seed=9), "d4t", rounds=2, budget_s=1e-9)
