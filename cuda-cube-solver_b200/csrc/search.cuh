@@ -37,7 +37,8 @@ struct alignas(16) Slot {
     uint32_t table;                  // 0: the handle's table, 1: its second resident table
     uint32_t queued;                 // QUEUED | gen while the work ring holds a live entry for this cube
     uint32_t gen;                    // generation of the slot (server: incremented on every reuse)
-    uint32_t pad2[1];
+    uint32_t failed;                 // a subtree of the current iteration was dropped: without a solution in it
+                                     // the cube ends as SLOT_ERROR, never with a longer one
 };
 
 struct QueueState {

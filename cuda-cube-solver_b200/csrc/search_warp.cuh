@@ -31,6 +31,9 @@ namespace ccs {
 #define CCS_WARP_POOL 32
 #define CCS_WARP_STACK 6
 #endif
+#ifndef CCS_WARP_SPILL
+#define CCS_WARP_SPILL 32
+#endif
 
 constexpr uint32_t WN_E2 = 24;      // frame k: c0 c1 e0 e1 at 4k, e2 here + k
 constexpr uint32_t WN_H = 30;       // bounds, 5 bits per frame
@@ -48,7 +51,7 @@ constexpr uint32_t WARP_WIDE = 11;  // budgets held to be wide before they are c
 constexpr uint32_t WARP_BARREN = 1u << 16;  // passes without a probe or a poll after which a warp gives up
 constexpr uint32_t WARP_HOLD = 2048;  // passes (about 10 ms) after which a warp takes its next item from the
                                       // queue again, so that a long iteration does not keep warps from others
-constexpr int WARP_SPILL = 32;      // spilled nodes per lane
+constexpr int WARP_SPILL = CCS_WARP_SPILL;  // spilled nodes per lane
 
 __device__ __forceinline__ State node_frame(const uint32_t* n, uint32_t k) {
     const Word4 a = reinterpret_cast<const Word4*>(n)[k];
@@ -303,12 +306,13 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_warp(const WarpTa
                 // free entry: the shallowest ones go to the spill list.
                 for (uint32_t i = 0; i < 16u && ns; ++i) {
                     const uint32_t best = shallowest(), owner = (best >> 3) & 31u, j = best & 7u;
-                    if (spilled >= 32u * WARP_SPILL) {
-                        if (lane == 0) atomicOr(&P.q->error, ERR_STACK);
-                    } else if (lane == (spilled & 31u)) {
-                        pack_entry(owner, j, sw1[spilled >> 5], sw2[spilled >> 5], sw3[spilled >> 5]);
+                    if (spilled < 32u * WARP_SPILL) {
+                        if (lane == (spilled & 31u)) pack_entry(owner, j, sw1[spilled >> 5], sw2[spilled >> 5], sw3[spilled >> 5]);
+                        ++spilled;
+                    } else if (lane == 0) {  // the subtree is dropped: this iteration cannot prove its bound
+                        atomicOr(&P.q->error, ERR_STACK);
+                        atomicExch(&P.slots[slot].failed, 1u);
                     }
-                    ++spilled;
                     if (lane == owner) mine |= 31u << (5u * j), refs[stash[64u * j + 32u + lane] & 63u] -= 1u;
                     --ns;
                     __syncwarp();
@@ -473,6 +477,8 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_warp(const WarpTa
                             __threadfence();
                             if (*(volatile uint32_t*)&sl.found) {
                                 finish_slot(P, slot, SLOT_SOLVED);
+                            } else if (*(volatile uint32_t*)&sl.failed) {
+                                finish_slot(P, slot, SLOT_ERROR);
                             } else if (bound + 1u > MAX_BOUND) {
                                 atomicOr(&P.q->error, ERR_BOUND);
                                 finish_slot(P, slot, SLOT_ERROR);

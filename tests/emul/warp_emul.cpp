@@ -196,10 +196,10 @@ void emul_warp_decode_b3(const uint32_t* sectors, const uint32_t* entry, int n, 
 // Warp intrinsics that the last emul_warp_solve ran: its length in steps of the warp.
 uint64_t emul_warp_turns() { return arrived[0]; }
 
-// Solves n cubes (at most 8) with one warp on an all-zero table; `starving`: with shorter
-// prefixes, donating all the time.  lengths[n]; nodes[24 n]: per cube and bound.  Returns the error bits (-1: unfinished).
-int emul_warp_solve(const char* name, const uint32_t* words, int n, int starving, uint32_t* lengths, uint8_t* moves,
-                    uint64_t* nodes, uint64_t* donated) {
+// Searches n cubes (at most 8) with one warp on an all-zero table; `starving`: 1: with shorter prefixes,
+// donating all the time, 2: in items of one move, without donations.  status[n]; lengths[n]; nodes[24 n]: per cube and bound.  Returns the error bits.
+int emul_warp_search(const char* name, const uint32_t* words, int n, int starving, uint32_t* status, uint32_t* lengths,
+                     uint8_t* moves, uint64_t* nodes, uint64_t* donated) {
     KindDesc kd;
     if (!preset_kind(name, &kd)) return -2;
     auto T = std::make_unique<DevImage>();
@@ -211,7 +211,7 @@ int emul_warp_solve(const char* name, const uint32_t* words, int n, int starving
     QueueState q;
     std::memset(&q, 0, sizeof q);
     std::memset(cells.data(), 0, sizeof(DonationCell) * cells.size());
-    q.starving = (uint32_t)starving;
+    q.starving = starving == 1;
     constexpr uint32_t CAP = 64;
     std::vector<unsigned long long> ring(5 * CAP + 64, ~0ull);
     std::vector<std::vector<uint32_t>> prefixes;
@@ -225,9 +225,10 @@ int emul_warp_solve(const char* name, const uint32_t* words, int n, int starving
     P.slots = slots.data(), P.q = &q, P.n_slots = (uint32_t)n;
     P.ring = ring.data(), P.ring_cap = 4 * CAP + 64, P.admit = ring.data() + P.ring_cap, P.admit_cap = CAP;
     P.classidx = corner_classes().classidx.data(), P.table = P.table2 = table.get();
-    P.base_plen = starving ? 3 : 4, P.max_plen = 4, P.few_divisor = 1, P.few_max_active = 4, P.shallow_min_active = 32;
+    P.base_plen = starving == 2 ? 1 : starving ? 3 : 4, P.max_plen = 4, P.few_divisor = 1, P.few_max_active = 4, P.shallow_min_active = 32;
     P.deeper_at[0] = P.deeper_at[1] = P.warp_many_at[0] = P.warp_many_at[1] = ~0ull;
     P.warp_items = 1, P.warp_at[0] = 200, P.warp_at[1] = 20000;  // prefixes two shorter, one, the base's
+    if (starving == 2) P.warp_at[0] = P.warp_at[1] = ~0ull;
     P.idle_limit = 1000, P.spread = 64;
     P.don = cells.data(), P.don_cap = 64, P.don_target = 8, P.don_min_depth = 2, P.don_period = 16;
     for (int i = 0; i < n; ++i) {
@@ -256,12 +257,21 @@ int emul_warp_solve(const char* name, const uint32_t* words, int n, int starving
     cur = 0;
     swapcontext(&main_ctx, &ctx[0]);
     for (int i = 0; i < n; ++i) {
-        if (slots[i].status != SLOT_SOLVED) return -1;
+        status[i] = slots[i].status;
         lengths[i] = slots[i].sol_len;
         std::memcpy(moves + 24 * i, slots[i].sol, 24);
         for (int b = 0; b < 24; ++b) nodes[24 * i + b] = slots[i].iter_nodes[b];
     }
     *donated = q.donated;
     return (int)q.error;
+}
+// The same for cubes that it is to solve (-1: one is unfinished).
+int emul_warp_solve(const char* name, const uint32_t* words, int n, int starving, uint32_t* lengths, uint8_t* moves,
+                    uint64_t* nodes, uint64_t* donated) {
+    std::vector<uint32_t> status(n);
+    const int error = emul_warp_search(name, words, n, starving, status.data(), lengths, moves, nodes, donated);
+    for (int i = 0; i < n; ++i)
+        if (status[i] != SLOT_SOLVED) return -1;
+    return error;
 }
 }

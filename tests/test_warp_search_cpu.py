@@ -96,3 +96,24 @@ def test_items_of_a_solved_cube_are_dropped_together(libs):
     assert libs["full"].emul_warp_solve(b"s4", ptr[0], 1, 0, ptr[1], ptr[2], ptr[3], ctypes.byref(donated)) == 0
     libs["full"].emul_warp_turns.restype = ctypes.c_uint64
     assert length[0] == 5 and libs["full"].emul_warp_turns() < 20 * len(canonical_prefixes(4))
+
+
+SLOT_SOLVED, SLOT_ERROR, ERR_STACK = 2, 3, 4
+
+
+@pytest.mark.parametrize("back", [[17, 13, 8, 3], [17, 13, 8, 3, 0, 5, 16]])
+def test_a_full_spill_list_fails_the_cube(libs, back):
+    """With room for 32 spilled nodes an iteration of four moves drops subtrees: the cube ends there as an error,
+    it is not searched on for a longer solution.  One found in that iteration all the same is optimal."""
+
+    state = apply_moves(CubieState(), [MOVES_HTM[3 * (m // 3) + 2 - m % 3] for m in reversed(back)])
+    lib = ctypes.CDLL(str(ROOT / "_build" / "emul" / "libccs_warp_over.so"))
+    words, status, length, moves = state_words([state]), np.zeros(1, np.uint32), np.zeros(1, np.uint32), np.zeros(24, np.uint8)
+    nodes, donated = np.zeros(24, np.uint64), ctypes.c_uint64()
+    ptr = [ctypes.c_void_p(a.ctypes.data) for a in (words, status, length, moves, nodes)]
+    assert lib.emul_warp_search(b"s4", ptr[0], 1, 2, *ptr[1:], ctypes.byref(donated)) == ERR_STACK
+    if len(back) > 4 or status[0] != SLOT_SOLVED:
+        assert status[0] == SLOT_ERROR
+    else:
+        assert length[0] == 4
+    assert nodes[4] > 0 and nodes[5:].sum() == 0
