@@ -34,6 +34,9 @@ namespace ccs {
 #ifndef CCS_WARP_SPILL
 #define CCS_WARP_SPILL 32
 #endif
+#ifndef CCS_WARP_BARREN
+#define CCS_WARP_BARREN (1u << 16)
+#endif
 
 constexpr uint32_t WN_E2 = 24;      // frame k: c0 c1 e0 e1 at 4k, e2 here + k
 constexpr uint32_t WN_H = 30;       // bounds, 5 bits per frame
@@ -48,7 +51,8 @@ constexpr uint32_t WARP_QUEUE = 256;              // children of open nodes (nod
 constexpr uint32_t WARP_WORDS = WN_POOL * WN_STRIDE + 64u * WARP_STACK + WARP_QUEUE / 2u + 96u;  // shared memory of a warp
 constexpr uint32_t WARP_RATIO = 4, WARP_COOL = 4;  // see OPEN
 constexpr uint32_t WARP_WIDE = 11;  // budgets held to be wide before they are counted (most entries are 11 or less)
-constexpr uint32_t WARP_BARREN = 1u << 16;  // passes without a probe or a poll after which a warp gives up
+constexpr uint32_t WARP_BARREN = CCS_WARP_BARREN;  // passes without a probe or a poll after which a warp gives
+                                                   // its work up
 constexpr uint32_t WARP_HOLD = 2048;  // passes (about 10 ms) after which a warp takes its next item from the
                                       // queue again, so that a long iteration does not keep warps from others
 constexpr int WARP_SPILL = CCS_WARP_SPILL;  // spilled nodes per lane
@@ -154,6 +158,10 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_warp(const WarpTa
         used = __reduce_or_sync(FULL, used);
         return __ballot_sync(FULL, refs[lane] == 0u) & ~used & POOL_ALL;
     };
+    // Everything the warp holds is dropped; its units only count as done.
+    auto drop_all = [&]() {
+        ns = spilled = 0, mine = NONE, head = tail, refs[lane] = 0u, dry = true, ch[0].k = ch[1].k = 7u;
+    };
     // A stash entry (bounds; node | move << 6 | children << 11)
     // ... as a node of its own: bounds | depth << 32 | budget << 37 | children << 42 | prefix
     // length << 60, and its path.
@@ -257,7 +265,7 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_warp(const WarpTa
             look = __ballot_sync(FULL, look != 0u);
             if (handed[lane] >= 1u << 20) handed[lane] >>= 1, passed[lane] >>= 1;  // (counts of late)
             wide_at = __ballot_sync(FULL, handed[lane] < 16u ? lane >= WARP_WIDE : WARP_RATIO * passed[lane] >= handed[lane]);
-            if (look & 3u) ns = spilled = 0, mine = NONE, head = tail, refs[lane] = 0u, dry = true, ch[0].k = ch[1].k = 7u;
+            if (look & 3u) drop_all();
             if ((look & 12u) == 4u && lane == 0u) ((volatile QueueState*)P.q)->starving = 0u;  // enough wait
             // DONATE the shallowest stashed child while warps starve (the rule of search_phased.cuh).
             uint32_t give = 0;
@@ -282,14 +290,18 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_warp(const WarpTa
             }
         }
 
-        const uint32_t idle0 = __ballot_sync(FULL, ch[0].k == 7u), idle1 = __ballot_sync(FULL, ch[1].k == 7u);
-        const uint32_t n_idle = __popc(idle0) + __popc(idle1);
         const uint32_t probing = __popc(__ballot_sync(FULL, ch[0].k < 6u)) + __popc(__ballot_sync(FULL, ch[1].k < 6u));
         barren = probing ? 0u : barren + 1u;
         if (barren > WARP_BARREN) {  // (never reached: a warp that makes no probe has work to finish or polls)
-            if (lane == 0) atomicOr(&P.q->error, ERR_STUCK);
-            break;
+            if (lane == 0) {
+                atomicOr(&P.q->error, ERR_STUCK);
+                atomicExch(&P.slots[slot].failed, 1u);
+            }
+            drop_all();
+            barren = 0;
         }
+        const uint32_t idle0 = __ballot_sync(FULL, ch[0].k == 7u), idle1 = __ballot_sync(FULL, ch[1].k == 7u);
+        const uint32_t n_idle = __popc(idle0) + __popc(idle1);
 
         // OPEN up to five stashed children, the deepest first, when fewer children are queued than
         // there are places for: six lanes build a node's frames and queue its children.  A wide node

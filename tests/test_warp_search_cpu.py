@@ -98,7 +98,7 @@ def test_items_of_a_solved_cube_are_dropped_together(libs):
     assert length[0] == 5 and libs["full"].emul_warp_turns() < 20 * len(canonical_prefixes(4))
 
 
-SLOT_SOLVED, SLOT_ERROR, ERR_STACK = 2, 3, 4
+SLOT_SOLVED, SLOT_ERROR, ERR_STACK, ERR_STUCK = 2, 3, 4, 8
 
 
 @pytest.mark.parametrize("back", [[17, 13, 8, 3], [17, 13, 8, 3, 0, 5, 16]])
@@ -117,3 +117,16 @@ def test_a_full_spill_list_fails_the_cube(libs, back):
     else:
         assert length[0] == 4
     assert nodes[4] > 0 and nodes[5:].sum() == 0
+
+
+def test_a_warp_that_gives_up_fails_the_cube(libs):
+    """A warp that makes no progress drops its work and counts its units as done, so that the cube ends in an
+    error (a served one would otherwise never end)."""
+
+    lib = ctypes.CDLL(str(ROOT / "_build" / "emul" / "libccs_warp_stuck.so"))
+    state = workloads.scramble_state(workloads.small_scrambles(1, seed=5)[0])
+    words, status, length, moves = state_words([state]), np.zeros(1, np.uint32), np.zeros(1, np.uint32), np.zeros(24, np.uint8)
+    nodes, donated = np.zeros(24, np.uint64), ctypes.c_uint64()
+    ptr = [ctypes.c_void_p(a.ctypes.data) for a in (words, status, length, moves, nodes)]
+    assert lib.emul_warp_search(b"s4", ptr[0], 1, 0, *ptr[1:], ctypes.byref(donated)) == ERR_STUCK
+    assert status[0] == SLOT_ERROR
