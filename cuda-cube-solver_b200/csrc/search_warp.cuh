@@ -34,6 +34,9 @@ namespace ccs {
 #ifndef CCS_WARP_SPILL
 #define CCS_WARP_SPILL 32
 #endif
+#ifndef CCS_WARP_FULL
+#define CCS_WARP_FULL (CCS_WARP_SPILL > 8 ? 32u * CCS_WARP_SPILL - 248u : 0u)
+#endif
 #ifndef CCS_WARP_BARREN
 #define CCS_WARP_BARREN (1u << 16)
 #endif
@@ -56,6 +59,11 @@ constexpr uint32_t WARP_BARREN = CCS_WARP_BARREN;  // passes without a probe or 
 constexpr uint32_t WARP_HOLD = 2048;  // passes (about 10 ms) after which a warp takes its next item from the
                                       // queue again, so that a long iteration does not keep warps from others
 constexpr int WARP_SPILL = CCS_WARP_SPILL;  // spilled nodes per lane
+// Children stashed or spilled from which on a warp searches one child at a time, so that the spill list
+// cannot overflow.  Up to here at most 64 children are under evaluation and 138 queued (63 and five nodes of 15),
+// which may all pass; beyond, the deepest child is opened alone, one of its children at a time, and stays where
+// it is until they are through, which adds at most one to each of 22 depths.
+constexpr uint32_t WARP_FULL = CCS_WARP_FULL;
 
 __device__ __forceinline__ State node_frame(const uint32_t* n, uint32_t k) {
     const Word4 a = reinterpret_cast<const Word4*>(n)[k];
@@ -310,11 +318,12 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_warp(const WarpTa
         // and more of them opened meanwhile would turn the search breadth-first and fill the stash.
         ++cool;
         const uint32_t supply = tail - head;
-        if (ns && (supply < n_idle || !probing)) {
+        const bool full = ns + spilled > WARP_FULL;
+        if (ns && (full ? !probing && !supply : supply < n_idle || !probing)) {
             uint32_t room = free_places();
-            if (!probing && (!room || supply > WARP_QUEUE - 96u) && (!n_idle || !supply)) {
+            if (!probing && (!room || supply >= 64u || (full && n_idle < 64u)) && (!n_idle || !supply)) {
                 // Nothing is on its way and nothing can be opened -- every place holds the parent of a
-                // stashed or queued child, or the queue is full and no lane with a passed child has a
+                // stashed or queued child, or enough are queued and no lane with a passed child has a
                 // free entry: the shallowest ones go to the spill list.
                 for (uint32_t i = 0; i < 16u && ns; ++i) {
                     const uint32_t best = shallowest(), owner = (best >> 3) & 31u, j = best & 7u;
@@ -332,11 +341,11 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_warp(const WarpTa
                 room = free_places();
             }
             const bool open_wide = (cool >= WARP_COOL && supply < 64u) || (!supply && probing < 32u) || !probing;
-            const uint32_t most = supply > WARP_QUEUE - 96u ? 0u : min((uint32_t)__popc(room), 5u);
+            const uint32_t most = supply >= 64u || (full && n_idle < 64u) ? 0u : min((uint32_t)__popc(room), full ? 1u : 5u);
             const uint32_t best = deepest(), level = best >> 3;
-            const bool wide = level == 31u || ((wide_at >> level) & 1u);
+            const bool wide = level == 31u || (!full && ((wide_at >> level) & 1u));
             const uint32_t low = __reduce_min_sync(FULL, wide ? 31u : level);  // deepest narrow one
-            uint32_t take = __ballot_sync(FULL, !wide && level <= low + 1u);
+            uint32_t take = __ballot_sync(FULL, !wide && level <= low + (full ? 0u : 1u));
             if ((uint32_t)__popc(take) < most) take = __ballot_sync(FULL, !wide);
             uint32_t cnt = 0, from = 0, to = 0;
 #pragma unroll
@@ -360,7 +369,7 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_warp(const WarpTa
                 }
             }
             const uint32_t entry = __shfl_sync(FULL, best, from) & 7u;
-            uint32_t todo = 0, h = 0, budget = 0;
+            uint32_t todo = 0, h = 0, budget = 0, rest = 0;  // rest: children that wait for this one's, see WARP_FULL
             if (team < cnt) {
                 const uint32_t e1 = stash[64u * entry + 32u + from], mv = (e1 >> 6) & 31u;
                 const uint32_t* a = pool + (e1 & 63u) * WN_STRIDE;
@@ -368,6 +377,7 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_warp(const WarpTa
                 set_node_frame(b, tk, warp_step(T, node_frame(a, tk), tk, mv));
                 const uint32_t meta = a[WN_META], g = (meta >> 8) & 255u;
                 todo = e1 >> 11;
+                if (full) rest = todo & (todo - 1u), todo ^= rest;
                 h = stash[64u * entry + from];
                 budget = (meta & 255u) - 1u;
                 if (tk < 4u) {
@@ -378,7 +388,17 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_warp(const WarpTa
                     b[WN_H] = h;
                 } else {
                     b[WN_META] = meta + 255u;  // one move deeper, one less to the bound
-                    atomicSub(&refs[e1 & 63u], 1u);
+                    if (!rest) atomicSub(&refs[e1 & 63u], 1u);
+                }
+            }
+            if (full) {  // (one was opened at most: what is left of it stays in its lane's stash)
+                const uint32_t owner = __shfl_sync(FULL, from, 0);
+                rest = __shfl_sync(FULL, rest, 0);
+                __syncwarp();
+                if (rest && lane == owner) {
+                    uint32_t* e1 = stash + 64u * (best & 7u) + 32u + lane;
+                    *e1 = (*e1 & 0x7FFu) | (rest << 11);
+                    mine ^= (31u ^ level) << (5u * (best & 7u));
                 }
             }
             // frame order, a frame per lane: at the bound, one below, the rest
@@ -406,7 +426,7 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_warp(const WarpTa
                 pool[to * WN_STRIDE + WN_ORD] = at_edge | (below_it << 6) | ((~(at_edge | below_it) & 63u) << 12) | ((budget - 1u) << 18);
             }
             tail += all;
-            ns -= cnt;
+            ns -= rest ? 0u : cnt;
             __syncwarp();
         }
 
@@ -445,13 +465,19 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_warp(const WarpTa
             uint32_t build = 0;
             const bool all_idle = left == 64u;
             if (spilled) {
-                if (free_places()) {
-                    --spilled;
-                    const int l = (int)(spilled & 31u), i = (int)(spilled >> 5);
+                if ((!full || all_idle) && free_places()) {
+                    const int l = (int)((spilled - 1u) & 31u), i = (int)((spilled - 1u) >> 5);
                     w1 = __shfl_sync(FULL, sw1[i], l);
                     w2 = __shfl_sync(FULL, sw2[i], l);
                     w3 = __shfl_sync(FULL, sw3[i], l);
                     build = 1;
+                    const uint32_t kids = (uint32_t)(w1 >> 42) & 0x3FFFFu, rest = full ? kids & (kids - 1u) : 0u;
+                    if (rest) {
+                        if (lane == (uint32_t)l) sw1[i] ^= (unsigned long long)(kids ^ rest) << 42;
+                        w1 ^= (unsigned long long)rest << 42;
+                    } else {
+                        --spilled;
+                    }
                 }
             } else if (held && !dry && free_places()) {
                 uint32_t idx = 0, plen = 0, ok = 0;

@@ -130,3 +130,19 @@ def test_a_warp_that_gives_up_fails_the_cube(libs):
     ptr = [ctypes.c_void_p(a.ctypes.data) for a in (words, status, length, moves, nodes)]
     assert lib.emul_warp_search(b"s4", ptr[0], 1, 0, *ptr[1:], ctypes.byref(donated)) == ERR_STUCK
     assert status[0] == SLOT_ERROR
+
+
+def test_a_nearly_full_spill_list_narrows_the_search(libs):
+    """With room for 96 spilled nodes and one child at a time from 10 on, a search that would hold more than 96 (the
+    list overflows without that rule) keeps within its list and still visits every node once."""
+
+    back = [17, 13, 8, 3]
+    state = apply_moves(CubieState(), [MOVES_HTM[3 * (m // 3) + 2 - m % 3] for m in reversed(back)])
+    lib = ctypes.CDLL(str(ROOT / "_build" / "emul" / "libccs_warp_narrow.so"))
+    words, status, length, moves = state_words([state]), np.zeros(1, np.uint32), np.zeros(1, np.uint32), np.zeros(24, np.uint8)
+    nodes, donated = np.zeros(24, np.uint64), ctypes.c_uint64()
+    ptr = [ctypes.c_void_p(a.ctypes.data) for a in (words, status, length, moves, nodes)]
+    assert lib.emul_warp_search(b"s4", ptr[0], 1, 2, *ptr[1:], ctypes.byref(donated)) == 0
+    assert status[0] == SLOT_SOLVED and length[0] == 4
+    count = np.cumsum([len(canonical_prefixes(L)) for L in range(1, 4)])  # (items of one move)
+    assert nodes[1:4].tolist() == count.tolist()
