@@ -6,6 +6,7 @@
 namespace ccs {
 
 constexpr uint32_t SLOT_FREE = 0, SLOT_ACTIVE = 1, SLOT_SOLVED = 2, SLOT_ERROR = 3;
+constexpr uint32_t FOUND_FAILED = 2;
 constexpr unsigned long long TICKET_IDLE = 0x7FFFFFFFull;  // ticket of a slot with no iteration: exhausted
 constexpr int MAX_PLEN = 6;
 constexpr uint32_t RING_RETIRED = 0xFFFFFFFFu;  // ring entry whose iteration is fully handed out
@@ -27,7 +28,8 @@ struct alignas(16) Slot {
     uint32_t open;                   // work units of the current epoch not yet finished: its items,
                                      // plus subtrees donated by lanes still holding a unit (so it
                                      // reaches 0 exactly when the epoch's last unit finishes)
-    uint32_t found;                  // set by the first lane that finds a solution
+    uint32_t found;                  // 1: set by the first lane that finds a solution; FOUND_FAILED: a subtree was
+                                     // dropped before, so the cube ends as SLOT_ERROR, never with a longer one
     uint32_t sol_len;
     uint32_t request;                // caller's tag (server request id)
     uint8_t sol[24];
@@ -37,8 +39,7 @@ struct alignas(16) Slot {
     uint32_t table;                  // 0: the handle's table, 1: its second resident table
     uint32_t queued;                 // QUEUED | gen while the work ring holds a live entry for this cube
     uint32_t gen;                    // generation of the slot (server: incremented on every reuse)
-    uint32_t failed;                 // a subtree of the current iteration was dropped: without a solution in it
-                                     // the cube ends as SLOT_ERROR, never with a longer one
+    uint32_t pad2[1];
 };
 
 struct QueueState {

@@ -35,7 +35,7 @@ namespace ccs {
 #define CCS_WARP_SPILL 32
 #endif
 #ifndef CCS_WARP_FULL
-#define CCS_WARP_FULL (CCS_WARP_SPILL > 8 ? 32u * CCS_WARP_SPILL - 248u : 0u)
+#define CCS_WARP_FULL (CCS_WARP_SPILL > 10 ? 32u * CCS_WARP_SPILL - 324u : 0u)
 #endif
 #ifndef CCS_WARP_BARREN
 #define CCS_WARP_BARREN (1u << 16)
@@ -59,10 +59,10 @@ constexpr uint32_t WARP_BARREN = CCS_WARP_BARREN;  // passes without a probe or 
 constexpr uint32_t WARP_HOLD = 2048;  // passes (about 10 ms) after which a warp takes its next item from the
                                       // queue again, so that a long iteration does not keep warps from others
 constexpr int WARP_SPILL = CCS_WARP_SPILL;  // spilled nodes per lane
-// Children stashed or spilled from which on a warp searches one child at a time, so that the spill list
-// cannot overflow.  Up to here at most 64 children are under evaluation and 138 queued (63 and five nodes of 15),
-// which may all pass; beyond, the deepest child is opened alone, one of its children at a time, and stays where
-// it is until they are through, which adds at most one to each of 22 depths.
+// Children stashed or spilled from which on a warp opens no more of them, so that the spill list cannot
+// overflow.  Up to here at most 64 children are under evaluation and 235 queued (160 and five nodes of 15), which
+// may all pass.  Beyond, all of them go to the list, and the last one of the list is searched alone, one of its
+// children at a time: what is left of it waits in its place, which adds at most one node to each of 22 depths.
 constexpr uint32_t WARP_FULL = CCS_WARP_FULL;
 
 __device__ __forceinline__ State node_frame(const uint32_t* n, uint32_t k) {
@@ -117,6 +117,18 @@ __device__ __forceinline__ void admit_slot_warp(const WarpTables& T, const Searc
     __syncwarp();
 }
 
+// A warp leaves with units in hand: the cube ends as SLOT_ERROR (unless another warp has solved it).
+static __device__ __noinline__ void give_up(const SearchParams& P, uint32_t slot, uint32_t held) {
+    Slot& sl = P.slots[slot];
+    atomicOr(&P.q->error, ERR_STUCK);
+    atomicCAS(&sl.found, 0u, FOUND_FAILED);
+    __threadfence();
+    if (atomicSub(&sl.open, held) == held) {
+        __threadfence();
+        finish_slot(P, slot, *(volatile uint32_t*)&sl.found == FOUND_FAILED ? SLOT_ERROR : SLOT_SOLVED);
+    }
+}
+
 // Up to two children per lane are under evaluation.  k: frame to probe next, 6 = passed (see PUSH),
 // 7 = none.  budget: moves the child leaves to the bound.
 struct WarpChild {
@@ -124,7 +136,8 @@ struct WarpChild {
 };
 
 template <int MODE, int NEC, int FMT, int THREADS, int MINB>
-__global__ void __launch_bounds__(THREADS, MINB) search_kernel_warp(const WarpTables* __restrict__ gT, SearchParams P) {
+__global__ void __launch_bounds__(THREADS, MINB)
+search_kernel_warp(const WarpTables* __restrict__ gT, SearchParams P) {
     __shared__ WarpTables T;
     extern __shared__ Word4 pool_smem[];
     stage_tables(T, gT);
@@ -165,10 +178,6 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_warp(const WarpTa
         for (uint32_t i = head + lane; (int)(tail - i) > 0; i += 32u) used |= 1u << (queue[i % WARP_QUEUE] & 31u);
         used = __reduce_or_sync(FULL, used);
         return __ballot_sync(FULL, refs[lane] == 0u) & ~used & POOL_ALL;
-    };
-    // Everything the warp holds is dropped; its units only count as done.
-    auto drop_all = [&]() {
-        ns = spilled = 0, mine = NONE, head = tail, refs[lane] = 0u, dry = true, ch[0].k = ch[1].k = 7u;
     };
     // A stash entry (bounds; node | move << 6 | children << 11)
     // ... as a node of its own: bounds | depth << 32 | budget << 37 | children << 42 | prefix
@@ -273,7 +282,7 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_warp(const WarpTa
             look = __ballot_sync(FULL, look != 0u);
             if (handed[lane] >= 1u << 20) handed[lane] >>= 1, passed[lane] >>= 1;  // (counts of late)
             wide_at = __ballot_sync(FULL, handed[lane] < 16u ? lane >= WARP_WIDE : WARP_RATIO * passed[lane] >= handed[lane]);
-            if (look & 3u) drop_all();
+            if (look & 3u) ns = spilled = 0, mine = NONE, head = tail, refs[lane] = 0u, dry = true, ch[0].k = ch[1].k = 7u;
             if ((look & 12u) == 4u && lane == 0u) ((volatile QueueState*)P.q)->starving = 0u;  // enough wait
             // DONATE the shallowest stashed child while warps starve (the rule of search_phased.cuh).
             uint32_t give = 0;
@@ -298,18 +307,14 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_warp(const WarpTa
             }
         }
 
+        const uint32_t idle0 = __ballot_sync(FULL, ch[0].k == 7u), idle1 = __ballot_sync(FULL, ch[1].k == 7u);
+        const uint32_t n_idle = __popc(idle0) + __popc(idle1);
         const uint32_t probing = __popc(__ballot_sync(FULL, ch[0].k < 6u)) + __popc(__ballot_sync(FULL, ch[1].k < 6u));
         barren = probing ? 0u : barren + 1u;
         if (barren > WARP_BARREN) {  // (never reached: a warp that makes no probe has work to finish or polls)
-            if (lane == 0) {
-                atomicOr(&P.q->error, ERR_STUCK);
-                atomicExch(&P.slots[slot].failed, 1u);
-            }
-            drop_all();
-            barren = 0;
+            if (lane == 0) give_up(P, slot, held);
+            break;
         }
-        const uint32_t idle0 = __ballot_sync(FULL, ch[0].k == 7u), idle1 = __ballot_sync(FULL, ch[1].k == 7u);
-        const uint32_t n_idle = __popc(idle0) + __popc(idle1);
 
         // OPEN up to five stashed children, the deepest first, when fewer children are queued than
         // there are places for: six lanes build a node's frames and queue its children.  A wide node
@@ -319,12 +324,12 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_warp(const WarpTa
         ++cool;
         const uint32_t supply = tail - head;
         const bool full = ns + spilled > WARP_FULL;
-        if (ns && (full ? !probing && !supply : supply < n_idle || !probing)) {
+        if (ns && (supply < n_idle || !probing)) {
             uint32_t room = free_places();
-            if (!probing && (!room || supply >= 64u || (full && n_idle < 64u)) && (!n_idle || !supply)) {
+            if (!probing && (!room || supply > WARP_QUEUE - 96u || full) && (!n_idle || !supply)) {
                 // Nothing is on its way and nothing can be opened -- every place holds the parent of a
-                // stashed or queued child, or enough are queued and no lane with a passed child has a
-                // free entry: the shallowest ones go to the spill list.
+                // stashed or queued child, or the queue is full and no lane with a passed child has a
+                // free entry, or see WARP_FULL: the shallowest ones go to the spill list.
                 for (uint32_t i = 0; i < 16u && ns; ++i) {
                     const uint32_t best = shallowest(), owner = (best >> 3) & 31u, j = best & 7u;
                     if (spilled < 32u * WARP_SPILL) {
@@ -332,7 +337,7 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_warp(const WarpTa
                         ++spilled;
                     } else if (lane == 0) {  // the subtree is dropped: this iteration cannot prove its bound
                         atomicOr(&P.q->error, ERR_STACK);
-                        atomicExch(&P.slots[slot].failed, 1u);
+                        atomicCAS(&P.slots[slot].found, 0u, FOUND_FAILED);
                     }
                     if (lane == owner) mine |= 31u << (5u * j), refs[stash[64u * j + 32u + lane] & 63u] -= 1u;
                     --ns;
@@ -341,11 +346,11 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_warp(const WarpTa
                 room = free_places();
             }
             const bool open_wide = (cool >= WARP_COOL && supply < 64u) || (!supply && probing < 32u) || !probing;
-            const uint32_t most = supply >= 64u || (full && n_idle < 64u) ? 0u : min((uint32_t)__popc(room), full ? 1u : 5u);
+            const uint32_t most = supply > WARP_QUEUE - 96u || full ? 0u : min((uint32_t)__popc(room), 5u);
             const uint32_t best = deepest(), level = best >> 3;
-            const bool wide = level == 31u || (!full && ((wide_at >> level) & 1u));
+            const bool wide = level == 31u || ((wide_at >> level) & 1u);
             const uint32_t low = __reduce_min_sync(FULL, wide ? 31u : level);  // deepest narrow one
-            uint32_t take = __ballot_sync(FULL, !wide && level <= low + (full ? 0u : 1u));
+            uint32_t take = __ballot_sync(FULL, !wide && level <= low + 1u);
             if ((uint32_t)__popc(take) < most) take = __ballot_sync(FULL, !wide);
             uint32_t cnt = 0, from = 0, to = 0;
 #pragma unroll
@@ -369,7 +374,7 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_warp(const WarpTa
                 }
             }
             const uint32_t entry = __shfl_sync(FULL, best, from) & 7u;
-            uint32_t todo = 0, h = 0, budget = 0, rest = 0;  // rest: children that wait for this one's, see WARP_FULL
+            uint32_t todo = 0, h = 0, budget = 0;
             if (team < cnt) {
                 const uint32_t e1 = stash[64u * entry + 32u + from], mv = (e1 >> 6) & 31u;
                 const uint32_t* a = pool + (e1 & 63u) * WN_STRIDE;
@@ -377,7 +382,6 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_warp(const WarpTa
                 set_node_frame(b, tk, warp_step(T, node_frame(a, tk), tk, mv));
                 const uint32_t meta = a[WN_META], g = (meta >> 8) & 255u;
                 todo = e1 >> 11;
-                if (full) rest = todo & (todo - 1u), todo ^= rest;
                 h = stash[64u * entry + from];
                 budget = (meta & 255u) - 1u;
                 if (tk < 4u) {
@@ -388,17 +392,7 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_warp(const WarpTa
                     b[WN_H] = h;
                 } else {
                     b[WN_META] = meta + 255u;  // one move deeper, one less to the bound
-                    if (!rest) atomicSub(&refs[e1 & 63u], 1u);
-                }
-            }
-            if (full) {  // (one was opened at most: what is left of it stays in its lane's stash)
-                const uint32_t owner = __shfl_sync(FULL, from, 0);
-                rest = __shfl_sync(FULL, rest, 0);
-                __syncwarp();
-                if (rest && lane == owner) {
-                    uint32_t* e1 = stash + 64u * (best & 7u) + 32u + lane;
-                    *e1 = (*e1 & 0x7FFu) | (rest << 11);
-                    mine ^= (31u ^ level) << (5u * (best & 7u));
+                    atomicSub(&refs[e1 & 63u], 1u);
                 }
             }
             // frame order, a frame per lane: at the bound, one below, the rest
@@ -426,7 +420,7 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_warp(const WarpTa
                 pool[to * WN_STRIDE + WN_ORD] = at_edge | (below_it << 6) | ((~(at_edge | below_it) & 63u) << 12) | ((budget - 1u) << 18);
             }
             tail += all;
-            ns -= rest ? 0u : cnt;
+            ns -= cnt;
             __syncwarp();
         }
 
@@ -472,7 +466,7 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_warp(const WarpTa
                     w3 = __shfl_sync(FULL, sw3[i], l);
                     build = 1;
                     const uint32_t kids = (uint32_t)(w1 >> 42) & 0x3FFFFu, rest = full ? kids & (kids - 1u) : 0u;
-                    if (rest) {
+                    if (rest) {  // (its other children wait for this one's)
                         if (lane == (uint32_t)l) sw1[i] ^= (unsigned long long)(kids ^ rest) << 42;
                         w1 ^= (unsigned long long)rest << 42;
                     } else {
@@ -513,10 +507,8 @@ __global__ void __launch_bounds__(THREADS, MINB) search_kernel_warp(const WarpTa
                         const bool final_unit = atomicSub(&sl.open, held) == held;
                         if (final_unit) {
                             __threadfence();
-                            if (*(volatile uint32_t*)&sl.found) {
-                                finish_slot(P, slot, SLOT_SOLVED);
-                            } else if (*(volatile uint32_t*)&sl.failed) {
-                                finish_slot(P, slot, SLOT_ERROR);
+                            if (const uint32_t found = *(volatile uint32_t*)&sl.found) {
+                                finish_slot(P, slot, found == FOUND_FAILED ? SLOT_ERROR : SLOT_SOLVED);
                             } else if (bound + 1u > MAX_BOUND) {
                                 atomicOr(&P.q->error, ERR_BOUND);
                                 finish_slot(P, slot, SLOT_ERROR);

@@ -22,6 +22,7 @@
 #define __global__
 #define __restrict__
 #define __launch_bounds__(...)
+#define __grid_constant__
 #define __shared__
 #define CCS_HOST_EMULATION 1
 using std::max;
