@@ -32,7 +32,7 @@ namespace ccs {
 #define CCS_WARP_STACK 6
 #endif
 #ifndef CCS_WARP_SPILL
-#define CCS_WARP_SPILL 32
+#define CCS_WARP_SPILL 24
 #endif
 #ifndef CCS_WARP_FULL
 #define CCS_WARP_FULL (CCS_WARP_SPILL > 10 ? 32u * CCS_WARP_SPILL - 324u : 0u)
@@ -58,7 +58,8 @@ constexpr uint32_t WARP_BARREN = CCS_WARP_BARREN;  // passes without a probe or 
                                                    // its work up
 constexpr uint32_t WARP_HOLD = 2048;  // passes (about 10 ms) after which a warp takes its next item from the
                                       // queue again, so that a long iteration does not keep warps from others
-constexpr int WARP_SPILL = CCS_WARP_SPILL;  // spilled nodes per lane
+constexpr int WARP_SPILL = CCS_WARP_SPILL;  // spilled nodes per lane (with 24 the launch's stacks, 56 MB, stay below
+                                            // the 57 MB of 256 x 2 lanes: a server's budget counts them)
 // Children stashed or spilled from which on a warp opens no more of them, so that the spill list cannot
 // overflow.  Up to here at most 64 children are under evaluation and 235 queued (160 and five nodes of 15), which
 // may all pass.  Beyond, all of them go to the list, and the last one of the list is searched alone, one of its
@@ -137,7 +138,7 @@ struct WarpChild {
 
 template <int MODE, int NEC, int FMT, int THREADS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB)
-search_kernel_warp(const WarpTables* __restrict__ gT, SearchParams P) {
+search_kernel_warp(const WarpTables* __restrict__ gT, const __grid_constant__ SearchParams P) {  // (else every thread copies it)
     __shared__ WarpTables T;
     extern __shared__ Word4 pool_smem[];
     stage_tables(T, gT);

@@ -79,3 +79,16 @@ def test_server_admits_by_device_memory(lengths_golden):
         h.server_stop()
     assert [got[i].length for i in range(len(cubes))] == [c["length"] for c in cubes]
     assert mem["budget_bytes"] == budget and 1 <= mem["peak_in_flight"] <= 6
+
+
+def test_default_server_asks_for_no_more_memory_than_the_lane_kernel():
+    """A budget that the server of one search per lane (variant 2, without the warp kernel's 23 KB of
+    constants) started within is still enough."""
+
+    h = resident_handle("d4t")
+    fixed = {}
+    for variant in (0, 2):
+        h.server_start_budget(64 << 30, native.solve_opts(variant=variant))
+        fixed[variant] = h.server_memory()["fixed_bytes"]
+        h.server_stop()
+    assert fixed[0] <= fixed[2] - 24_000
