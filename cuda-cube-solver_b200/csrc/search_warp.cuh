@@ -285,13 +285,17 @@ search_kernel_warp(const WarpTables* __restrict__ gT, const __grid_constant__ Se
             wide_at = __ballot_sync(FULL, handed[lane] < 16u ? lane >= WARP_WIDE : WARP_RATIO * passed[lane] >= handed[lane]);
             if (look & 3u) ns = spilled = 0, mine = NONE, head = tail, refs[lane] = 0u, dry = true, ch[0].k = ch[1].k = 7u;
             if ((look & 12u) == 4u && lane == 0u) ((volatile QueueState*)P.q)->starving = 0u;  // enough wait
-            // DONATE the shallowest stashed child while warps starve (the rule of search_phased.cuh).
-            uint32_t give = 0;
-            if ((look & 28u) == 28u && ns > 1u) {
-                const uint32_t best = shallowest(), owner = (best >> 3) & 31u, j = best & 7u;
+            // DONATE while warps starve (the rule of search_phased.cuh): the last spilled node, else the
+            // shallowest stashed child.  (Without the spilled ones a wide search ends on a few warps: the superflip on d4t
+            // with base_plen 3 took 3.8 s, with them 2.7.)
+            if ((look & 28u) == 28u && (ns > 1u || spilled)) {
+                const uint32_t best = shallowest(), j = best & 7u, at = spilled - 1u;
+                const uint32_t owner = spilled ? at & 31u : (best >> 3) & 31u;
+                uint32_t give = 0;
                 if (lane == owner) {
                     unsigned long long w1, w2, w3;
-                    pack_entry(owner, j, w1, w2, w3);
+                    if (spilled) w1 = sw1[at >> 5], w2 = sw2[at >> 5], w3 = sw3[at >> 5];
+                    else pack_entry(owner, j, w1, w2, w3);
                     const uint32_t hb = (uint32_t)w1 & 0x3FFFFFFFu, g = (uint32_t)(w1 >> 32) & 31u, budget = (uint32_t)(w1 >> 37) & 31u;
                     uint32_t hmax = 0;
 #pragma unroll
@@ -300,11 +304,13 @@ search_kernel_warp(const WarpTables* __restrict__ gT, const __grid_constant__ Se
                         atomicAdd(&P.slots[slot].open, 1u);  // before the post: the count never runs short
                         w1 = (w1 & ~((31ull << 37) | (15ull << 60))) | ((unsigned long long)bound << 37);
                         give = post_donation(P, seed0 + iter, slot, w1, w2, w3);
-                        if (give) mine |= 31u << (5u * j), refs[stash[64u * j + 32u + lane] & 63u] -= 1u;
-                        else atomicSub(&P.slots[slot].open, 1u);
+                        if (!give) atomicSub(&P.slots[slot].open, 1u);
+                        else if (!spilled) mine |= 31u << (5u * j), refs[stash[64u * j + 32u + lane] & 63u] -= 1u;
                     }
                 }
-                ns -= __shfl_sync(FULL, give, owner);
+                give = __shfl_sync(FULL, give, owner);
+                if (spilled) spilled -= give;
+                else ns -= give;
             }
         }
 
