@@ -92,3 +92,31 @@ def test_default_server_asks_for_no_more_memory_than_the_lane_kernel():
         fixed[variant] = h.server_memory()["fixed_bytes"]
         h.server_stop()
     assert fixed[0] <= fixed[2] - 24_000
+
+
+def test_few_slots_reused_over_many_laps_of_the_ring():
+    """Two slots and a work ring of 320 positions (a handle's smallest): 200 cubes after one another reuse each
+    slot 100 times and queue some 1,500 iterations, so the ring wraps several times with live entries in it."""
+
+    from cuda_cube_solver import workloads
+
+    h = native.Handle()
+    try:
+        h.build_table("304", "block", None, keep_resident=1)
+        states = [workloads.scramble_state(s) for s in workloads.small_scrambles(200, seed=11)]
+        words = state_words(states)
+        h.server_start(2)
+        ids = {h.server_submit(words[i]): i for i in range(len(states))}
+        got, t0 = {}, time.time()
+        while len(got) < len(states) and time.time() - t0 < 120:
+            for rid, r in h.server_poll(64):
+                got[ids[rid]] = r
+            time.sleep(0.002)
+        h.server_stop()
+        assert len(got) == len(states)
+        want = [r.length for r in h.solve(words, native.solve_opts(timeout_s=120))]
+        assert [got[i].length for i in range(len(states))] == want
+        for i, r in got.items():
+            assert apply_moves(states[i], [MOVES_HTM[m] for m in r.moves[: r.length]]) == CubieState()
+    finally:
+        h.close()
