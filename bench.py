@@ -388,15 +388,33 @@ def reference_arm(args, world: int, rank: int, local: int) -> None:
     print(json.dumps(out))
 
 
-def bfs_roofline(passes: list[dict], entries: int, peak_gbs: float, ceiling: float | None) -> dict:
-    """The table build's passes against their rooflines: algorithmic bytes of a pass = a byte per
-    entry (its distance planes read and written) + the 32-byte sectors read at neighbours and claimed;
-    these also against the random-sector ceiling."""
+def row_bytes(kind: str, entries: int) -> tuple[int, int]:
+    """Bytes of a kind's distance planes (four words a row of its columns) and of one frontier bit set (one)."""
+
+    from cuda_cube_solver import native
+
+    columns = 16 if kind == "304" else native.kind_info(kind)[0]
+    word = 4 if columns > 16 else 2 if columns > 8 else 1
+    return entries // columns * 4 * word, entries // columns * word
+
+
+def bfs_roofline(passes: list[dict], entries: int, peak_gbs: float, ceiling: float | None,
+                 planes: tuple[int, int] | None = None) -> dict:
+    """The table build's passes against their rooflines.  Algorithmic bytes, with ``planes`` (row_bytes): a
+    listed pass reads its entries and writes those it found (8 bytes each), and takes a 32-byte sector per
+    neighbour read and claimed; a dense pass reads the distance planes, reads one frontier and writes the
+    next (its neighbours' sectors come from blocks of frontier bits, mostly out of L2, and are reported as
+    sectors only).  Without ``planes``: a byte per entry and a sector per neighbour, in every pass."""
 
     rows = []
-    for p in passes:
+    for i, p in enumerate(passes):
         random = p["random_reads"] + p["claims"]
-        algo = entries + SECTOR * random
+        if planes is None:
+            algo = entries + SECTOR * random
+        elif p["forward"]:
+            algo = 8 * ((passes[i - 1]["found"] if i else 1) + p["found"]) + SECTOR * random
+        else:
+            algo = planes[0] + 2 * planes[1]
         rows.append({"depth": p["depth"], "dir": "fwd" if p["forward"] else "bwd", "found": p["found"],
                      "random_sectors": random, "seconds": p["seconds"], "algorithmic_gb": algo / 1e9,
                      "achieved_gb_s": algo / p["seconds"] / 1e9, "random_sectors_per_s": random / p["seconds"]})
@@ -412,9 +430,8 @@ def bfs_roofline(passes: list[dict], entries: int, peak_gbs: float, ceiling: flo
             # Neighbours come in whole blocks of frontier bits, many from L2: a rate above the DRAM
             # random-sector ceiling says so, it is not a fraction of it.
             out["random_rate_over_dram_random_ceiling"] = top["random_sectors_per_s"] / ceiling
-            out["note"] = ("random accesses costed as 32-byte sectors; a rate above the search's DRAM "
-                           "random-sector ceiling means most of them hit L2 (profiles/bfs_rows_304.md: "
-                           "DRAM bytes per pass)")
+            out["note"] = ("neighbour sectors are read as whole blocks of frontier bits: a rate above the search's "
+                           "DRAM random-sector ceiling means most of them hit L2")
     return out
 
 
@@ -655,7 +672,7 @@ def main_arm(args, world: int, rank: int, local: int) -> None:
            "table_build": {"kind": args.kind, "format": args.format, "gpu_seconds": solver.build_seconds,
                            "wall_s": build_wall_s, "entries": entries, "entries_per_s": entries / solver.build_seconds,
                            "table_bytes": h.table_bytes(), "depth_counts": solver.build_counts,
-                           "roofline": bfs_roofline(build_passes, entries, peak, ceiling)},
+                           "roofline": bfs_roofline(build_passes, entries, peak, ceiling, row_bytes(args.kind, entries))},
            "wall_s_per_step": statistics.mean(wall)}
     print(json.dumps(out))
     barrier(world)
