@@ -30,7 +30,7 @@ using namespace ccs;
 
 namespace ccs {
 void fill_params(ccs_handle* h, const ccs_solve_opts* o, SearchParams* P);
-int resolve_variant(const ccs_solve_opts* o, int cubes);
+int resolve_variant(const ccs_solve_opts* o);
 int grid_for(ccs_handle* h, const ccs_solve_opts* o, int variant);
 int launch_kernel(ccs_handle* h, const SearchParams& P, int grid, cudaStream_t stream, int variant);
 void make_slot(const uint32_t state[5], uint32_t request, uint32_t table, Slot* s);
@@ -186,7 +186,7 @@ extern "C" int ccs_solve_noalloc(ccs_handle* h, const uint32_t* states, int n, c
     CCS_CUDA_TRY(cudaMemcpyAsync(P.admit, D.admit, 8ull * n, cudaMemcpyHostToDevice, st));
     CCS_CUDA_TRY(cudaMemcpyAsync(&S->q, &q, sizeof q, cudaMemcpyHostToDevice, st));
 
-    const int variant = resolve_variant(opts, n);
+    const int variant = resolve_variant(opts);
     const int grid = grid_for(h, opts, variant);
     const double timeout = opts && opts->timeout_s > 0 ? opts->timeout_s : 0;
     auto t0 = std::chrono::steady_clock::now();

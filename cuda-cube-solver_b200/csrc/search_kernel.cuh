@@ -8,7 +8,8 @@
 // tight; an inverse frame on the move's own axis keeps its parent's value (same coset); frames
 // are probed at the budget edge first, one below next, the rest last.
 //
-// Execution (this library's own): every lane runs its own depth-first search over one work item
+// Execution (this library's own; the lane kernels here and in search_phased.cuh -- the default kernel,
+// search_warp.cuh, shares the queue): every lane runs its own depth-first search over one work item
 // (a cube and a canonical move prefix).  Per warp iteration each lane performs exactly one table
 // probe; control work (next child, push, pop, item fetch) runs between probes.  Work comes from
 // a device ring of cube slots: the ticket of a slot hands out the prefix items of its current

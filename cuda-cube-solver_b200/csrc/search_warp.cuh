@@ -13,12 +13,11 @@
 // pushes, pops and fetches run for a few lanes at a time, and a call of few cubes was 75,776 lanes
 // each alone on a subtree of very uneven size.  Here 59 of 64 places hold a child, control is
 // uniform, and 2,960 warps share an iteration's items and search a subtree 32 lanes wide.  Measured
-// on B200, d4t, cubes/s before (the lane kernels' defaults) and now: one cube per call 57 -> 165, 16 at a
-// time 131 -> 270, 100 at a time 179 -> 300, 1,024 at a time 334 -> 351; the superflip on d4 0.75 -> 0.53
-// s.  640 threads a block, one block an SM: 96 registers, and with 32 nodes a warp some 50 KB stay L1;
-// 512 threads (116 registers) gave 313 cubes/s at 1,024, 768 (80 registers, spills) 329.  The one
-// case it loses: a lone superflip on d4t, 73 G probes of a tree that hardly narrows, 2.6 -> 3.7 s (on d4,
-// where the flip rule sends it, it gains).
+// on B200, d4t, cubes/s before (the lane kernels' defaults) and now: one cube per call 57 -> 203, 16 at a
+// time 131 -> 299, 100 at a time 179 -> 354, 1,024 at a time 334 -> 418, 4,096 with 5% hard 235 -> 283; a lone
+// superflip on d4 0.65 -> 0.43 s, on d4t, 73 G probes of a tree that hardly narrows, 2.53-2.76 -> 2.45 s.
+// 640 threads a block, one block an SM: 92 registers, and with 32 nodes a warp some 50 KB stay L1; when
+// 640 threads gave 351 cubes/s at 1,024, 512 (116 registers) gave 313 and 768 (80 registers, spills) 329.
 #pragma once
 
 #include "search_kernel.cuh"

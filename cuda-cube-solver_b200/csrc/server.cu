@@ -24,7 +24,7 @@ using namespace ccs;
 
 namespace ccs {
 void fill_params(ccs_handle* h, const ccs_solve_opts* o, SearchParams* P);
-int resolve_variant(const ccs_solve_opts* o, int cubes);
+int resolve_variant(const ccs_solve_opts* o);
 int grid_for(ccs_handle* h, const ccs_solve_opts* o, int variant);
 int launch_kernel(ccs_handle* h, const SearchParams& P, int grid, cudaStream_t stream, int variant);
 void make_slot(const uint32_t state[5], uint32_t request, uint32_t table, Slot* s);
@@ -180,7 +180,7 @@ int kernel_footprint_kind(ccs_handle* h, int variant, size_t* local_bytes, int* 
 
 // The automatic server kernel is the solve calls' (variant 12).
 static int server_variant(const ccs_solve_opts* opts) {
-    return resolve_variant(opts, 0);
+    return resolve_variant(opts);
 }
 
 // Device memory the server holds whatever the number of cubes: resident tables, constants,
@@ -256,11 +256,12 @@ extern "C" int ccs_server_start(ccs_handle* h, int slots, const ccs_solve_opts* 
     s->P.n_slots = (uint32_t)slots;
     s->P.persistent = 1;
     // Served cubes keep the plain deeper thresholds: with the few-cube rule on, the served
-    // stream's p50 rose from 43 to 131 ms on B200 (it pays off for a lone batch or plain solve).
+    // stream's p50 rose from 43 to 131 ms on B200 with 256 x 2 lanes (it pays off for a lone batch or plain
+    // solve; variant 12 divides by 1 unless told otherwise).
     s->P.few_max_active = 0;
     s->P.idle_limit = 1u << 16;  // ~0.25 s of idle polling, then the launch ends (relaunched on demand)
-    // Served streams steal with whole idle warps asking (opts->steal 0 or 2; 1: any idle lane
-    // asks; < 0: off).  Measured on B200 (256 x 2 with lookahead; 90% uniform, 9% of length >= 18,
+    // Served streams of the lane kernels steal with whole idle warps asking (opts->steal 0 or 2; 1: any
+    // idle lane asks; < 0: off); in variant 12 a warp asks in any case.  Measured on B200 (256 x 2 with lookahead; 90% uniform, 9% of length >= 18,
     // 1% superflips): sustained 86.8-89.0 cubes/s at 100 requests/s with whole warps asking, 77.8
     // with any lane asking, 75.4 without stealing.
     if (!opts || opts->steal == 0) s->P.don_eager = 0u;

@@ -42,7 +42,7 @@ int ensure_search_buffers(ccs_handle* h, uint32_t slots) {
     return CCS_OK;
 }
 
-int resolve_variant(const ccs_solve_opts* o, int cubes);
+int resolve_variant(const ccs_solve_opts* o);
 
 void fill_params(ccs_handle* h, const ccs_solve_opts* o, SearchParams* P) {
     std::memset(P, 0, sizeof *P);
@@ -69,8 +69,8 @@ void fill_params(ccs_handle* h, const ccs_solve_opts* o, SearchParams* P) {
     P->shallow_at[0] = (unsigned long long)(o && o->shallow_at0 != 0 ? (o->shallow_at0 > 0 ? o->shallow_at0 : 0) : 1e5);
     P->shallow_at[1] = (unsigned long long)(o && o->shallow_at1 != 0 ? (o->shallow_at1 > 0 ? o->shallow_at1 : 0) : 1.5e6);
     P->shallow_min_active = 32;
-    // A lone 20-move cube on B200: deeper prefixes from 1e6 / 6e7 nodes instead of 5e7 / 3e9 took
-    // the superflip from 1.66 to 0.74 s on d4 and from 12.7 to 7.5 s on d4t.
+    // A lone 20-move cube on B200, searched by the lane kernels: deeper prefixes from 1e6 / 6e7 nodes instead
+    // of 5e7 / 3e9 took the superflip from 1.66 to 0.74 s on d4 and from 12.7 to 7.5 s on d4t.
     P->few_divisor = o && o->few_divisor > 0 ? (uint32_t)o->few_divisor : 50u;
     P->few_max_active = 4;  // (the server sets 0: see ccs_server_start)
     P->idle_limit = 1u << 21;  // ~8 s of idle polling (4 us back-off) before a warp leaves
@@ -87,8 +87,8 @@ void fill_params(ccs_handle* h, const ccs_solve_opts* o, SearchParams* P) {
     uint32_t period = o && o->steal_period > 0 ? (uint32_t)o->steal_period : 64u;
     while (period & (period - 1)) period &= period - 1;  // a power of two (rounded down)
     P->don_period = period;
-    // Any lane without work asks for donations (steal 0), or only whole idle warps (steal 2).
-    // Measured on B200 with 256 x 3: the 4,096-cube batch with 5% hard positions 220 against 194
+    // Any lane without work asks for donations (steal 0), or only whole idle warps (steal 2); the lane
+    // kernels read it.  Measured on B200 with 256 x 3: the 4,096-cube batch with 5% hard positions 220 against 194
     // cubes/s, a lone superflip on d4t 3.1 against 5.8 s, uniform batches within 4%.
     P->don_eager = o && o->steal == 2 ? 0u : 1u;
     P->don_min_prev = o && o->steal_min_nodes != 0 ? (o->steal_min_nodes > 0 ? (unsigned long long)o->steal_min_nodes : 0ull)
@@ -97,7 +97,7 @@ void fill_params(ccs_handle* h, const ccs_solve_opts* o, SearchParams* P) {
     // to begin with and grows with the last iteration's nodes -- an item of a few hundred nodes
     // keeps a warp busy past the walk to it, and 2,960 warps need some items each.  With many cubes
     // in flight other cubes fill the warps, and longer items cost fewer walks.
-    P->warp_items = resolve_variant(o, 0) == 12 ? 1u : 0u;
+    P->warp_items = resolve_variant(o) == 12 ? 1u : 0u;
     // (1,500: a lone cube's iteration after one of 3,400 nodes took 250 us with 243 items -- most warps had
     // none and the largest item was a long chain -- and 147 us with 3,240.  The second threshold stays: at
     // 60,000 the iteration after the next took 470 us against 410, 43,239 items being too many for it.)
@@ -127,9 +127,9 @@ void fill_params(ccs_handle* h, const ccs_solve_opts* o, SearchParams* P) {
 // 8 = sibling lookahead, 256 x 3; 9 = phase-ordered, 256 x 4 (32 warps per SM, 64 registers);
 // 10 = phase-ordered, 224 x 3 (21 warps, 96 registers); 11 = phase-ordered, 128 x 5 (20 warps, 96).
 // 12 = one search per warp (search_warp.cuh), 640 x 1.  0 = automatic: 12.  Measured on B200 (d4t,
-// cubes/s at one cube per call / 16 / 100 / 1,024 per call): 12 155 / 260 / 300 / 351, 2 58 / 131 /
+// cubes/s at one cube per call / 16 / 100 / 1,024 per call): 12 203 / 299 / 354 / 418, 2 58 / 131 /
 // 179 / 275, 3 44 / 125 / 162 / 334.
-int resolve_variant(const ccs_solve_opts* o, int cubes) {
+int resolve_variant(const ccs_solve_opts* o) {
     int v = o ? o->variant : 0;
     if (v <= 0 || v > 12) v = 12;
     return v;
@@ -231,7 +231,7 @@ extern "C" int ccs_solve_tables(ccs_handle* h, const uint32_t* states, const uin
     CCS_CUDA_TRY(cudaMemcpyAsync(P.admit, admit.data(), 8ull * n, cudaMemcpyHostToDevice, st));
     CCS_CUDA_TRY(cudaMemcpyAsync(h->d_q, &q, sizeof q, cudaMemcpyHostToDevice, st));
 
-    const int variant = resolve_variant(opts, n);
+    const int variant = resolve_variant(opts);
     const int grid = grid_for(h, opts, variant);
     const double timeout = opts && opts->timeout_s > 0 ? opts->timeout_s : 0;
     auto t0 = std::chrono::steady_clock::now();

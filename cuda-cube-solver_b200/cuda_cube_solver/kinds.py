@@ -213,8 +213,8 @@ class Preset:
     def build_bytes(self) -> int:
         """Device memory that building it here asks for: a byte per entry (padded to 16) and the encoded
         block table, plus the base-3 table while it is encoded from the block one.  (The build stays
-        within it: six or, past depth 14, seven bits' planes per entry while it searches, four or five
-        beside the tables.)"""
+        within it.  It holds six words a row of 8, 16 or 32 bits while it searches -- four distance planes and
+        two frontiers, 6 to 8 bits an entry -- and a seventh past depth 14; beside the tables, the planes alone.)"""
 
         depth = -(-self.entries // 16) * 16
         block = -(-self.entries // BLOCK_ENTRIES) * 32
