@@ -282,20 +282,23 @@ def verify_solutions(words: np.ndarray, solutions: list[list[int]]) -> bool:
     number of cubes, raise IndexError."""
 
     b = np.ascontiguousarray(words, np.uint32).reshape(-1, 5).view(np.uint8).reshape(-1, 20)
+    if len(solutions) == len(b) <= _CHECK_ONE_BY_ONE:
+        try:
+            solved = True
+            for state, moves in zip(b.tolist(), solutions):  # (all of them: a move above 17 is not in _STEPS)
+                for m in moves:
+                    if m >= 0:
+                        state = [becomes[state[src]] for src, becomes in _STEPS[m]]
+                solved = solved and state == _SOLVED
+            return solved
+        except TypeError:
+            pass  # moves that are no indices (3.0) are converted below
     if any(max(moves) >= 18 for moves in solutions if len(moves)):
         raise IndexError("a move is 0 to 17")
     if len(b) != len(solutions):
         if any(max(moves) >= 0 for moves in solutions if len(moves)):
             raise IndexError(f"moves for {len(solutions)} cubes, {len(b)} states")
         return bool((b == _SOLVED).all())
-    if len(b) <= _CHECK_ONE_BY_ONE:
-        for state, moves in zip(b.tolist(), solutions):
-            for m in moves:
-                if m >= 0:
-                    state = [becomes[state[src]] for src, becomes in _STEPS[int(m)]]
-            if state != _SOLVED:
-                return False
-        return True
     at = np.arange(20)
     for j in range(max((len(m) for m in solutions), default=0)):
         col = np.array([m[j] if j < len(m) and m[j] >= 0 else 18 for m in solutions]).astype(np.int64)
